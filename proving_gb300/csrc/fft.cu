@@ -14,8 +14,8 @@
 // of layers [lo, hi): every group of 2^(hi-lo) elements that differ only in
 // index bits [lo, hi) is independent for those layers. A CTA stages one tile —
 // such a group times 2^c neighbouring groups, chosen so global accesses are
-// contiguous runs — in shared memory, runs the layers as radix-8 register
-// stages, and writes the tile back. Evaluate's first pass reads each
+// contiguous runs — and runs the layers as two register stages of up to six
+// layers with an exchange in shared memory between them. Evaluate's first pass reads each
 // coefficient tile once from the (shorter) coefficient column: the
 // zero-padded top layers are identities, so every blown-up replica starts
 // from the same coefficients; replicas of a tile are adjacent CTAs and share
@@ -214,10 +214,8 @@ template <int T, bool OUTER>
 constexpr int tile_max_threads() {
   return OUTER ? 256 : (1 << (T / 2 + 3));
 }
-// Blocks per SM the register budget is sized for: tiles of up to 10 layers fit
-// four (64 registers) without spills, larger ones two. Four blocks keep more
-// tile loads in flight: the strided evaluate pass, which reads each coefficient
-// tile once for its replicas, is otherwise bound by its load latency.
+// Blocks per SM the register budget is sized for: the short tiles fit four
+// (64 registers) without spills, the 12-layer one two.
 template <int T, bool OUTER>
 constexpr int tile_min_blocks() {
   return T <= 10 ? 4 : 2;
@@ -353,6 +351,373 @@ __global__ void __launch_bounds__(tile_max_threads<T, OUTER>(), tile_min_blocks<
   }
 }
 
+// ---- passes of up to 10 layers: tiles go between global memory and registers directly ----
+//
+// The same two register stages, with less around them than fft_tile_kernel. A thread's first
+// stage loads its values straight from global memory and its last stage stores them straight from
+// registers wherever a warp's accesses are whole 32-byte sectors, so a strided pass touches shared
+// memory once (the exchange between its stages) behind one block barrier, and a contiguous pass,
+// whose groups of 2^T words belong to one warp each, needs no block barrier at all. Twiddles of the
+// table stages are loaded and doubled once per warp (one or a few words per lane) and read back as
+// broadcast 16-byte words.
+//
+// Bound: instruction issue. A butterfly is seven instructions and, alone in registers, 10.85 cycles
+// of a warp scheduler (the 64-bit product takes about two ALU slots beside its multiplier); the
+// passes run at 12.4 (contiguous) and 13.9-14.7 cycles a butterfly with DRAM 20-45% busy, against
+// 15.8-17.2 for tiles staged through shared memory on both sides of the stages (four block
+// barriers, twice the shared accesses, per-word address arithmetic). Measured, CUDA events:
+// 256 columns of 2^20 interpolate 1.33 -> 1.04 ms and evaluate onto 2^22 4.71 -> 3.69 ms; one
+// column of 2^24 138 -> 100 and 257 -> 178 us; 32 columns of 2^22 743 -> 640 and 1408 -> 1153 us.
+// Passes of 11 layers hold 64 values a thread (two stages of 5 and 6 layers, 512 threads an SM);
+// contiguous passes of up to 5 layers, strided ones of up to 3 and the 12-layer pass stay with
+// fft_tile_kernel (a 12-layer pass would need a third stage; 1000 columns of 2^12 measured 293 us
+// either way).
+
+__device__ __forceinline__ const uint32_t* layer_twiddles(const FftPass& p, uint32_t layer) {
+  return p.tw + ((1u << p.tw_log) - (1u << (p.tw_dom - layer)));
+}
+
+// The doubled twiddles of R layers from `layer0` up for the 2^R-value groups `group(k)`, k < n, as
+// tab[k 2^R + tw_off<R>(t) + q] = 2 tw[layer0 + t][(group << (R - 1 - t)) + q]. A lane's slot in a
+// group (hence its layer) is the same for every group it loads.
+template <int R, typename Group>
+__device__ __forceinline__ void fill_table(const FftPass& p, uint32_t layer0, uint32_t lane, int n, uint32_t* tab,
+                                           Group group) {
+#pragma unroll
+  for (uint32_t pos = lane & ((1u << R) - 1); pos + 1 < (1u << R); pos += (R > 5 ? 32 : 1 << R)) {
+    const uint32_t t = R - (32 - __clz((1u << R) - pos - 1));
+    const uint32_t* src = layer_twiddles(p, layer0 + t) + (pos - ((1u << R) - (1u << (R - t))));
+    for (int k = (int)(lane >> R); k < n; k += (R > 5 ? 1 : 32 >> R))
+      tab[(k << R) + pos] = __ldg(src + (group(k) << (R - 1 - t))) << 1;
+  }
+}
+
+// R layers on v with the doubled twiddles of one group's table.
+template <bool INV, int R>
+__device__ __forceinline__ void table_stage(uint32_t* v, const uint32_t* tab) {
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    const int t = INV ? k : R - 1 - k;
+    const int cnt = 1 << (R - 1 - t);
+#pragma unroll
+    for (int q0 = 0; q0 < cnt; q0 += 4) {
+      uint32_t w[4];
+      const uint32_t* src = tab + tw_off<R>(t) + q0;
+      if (cnt >= 4) {
+        const uint4 x = *reinterpret_cast<const uint4*>(src);
+        w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
+      } else {
+#pragma unroll
+        for (int q = 0; q < cnt; q++) w[q] = src[q];
+      }
+#pragma unroll
+      for (int q = 0; q < (cnt < 4 ? cnt : 4); q++) {
+#pragma unroll
+        for (int l = 0; l < (1 << t); l++) {
+          const int j = ((q0 + q) << (t + 1)) | l;
+          if (INV)
+            ibfly2(v[j], v[j | (1 << t)], w[q]);
+          else
+            bfly2(v[j], v[j | (1 << t)], w[q]);
+        }
+      }
+    }
+  }
+}
+
+// The lowest R >= 3 layers (circle layer included) on v = group g's 2^R consecutive values. The
+// circle layer's twiddles [y, -y, -x, x] come from the words (x, y) of line layer 1; a negated
+// twiddle swaps the butterfly's sum and difference instead.
+template <bool INV, int R>
+__device__ __forceinline__ void circle_stage(const FftPass& p, uint32_t g, uint32_t* v) {
+  static_assert(R >= 3 && R <= 5, "circle_stage");
+  uint32_t w[(1 << (R - 1)) - 1];  // line layer t >= 1 at offset 2^(R-1) - 2^(R-t)
+#pragma unroll
+  for (int t = 1; t < R; t++) {
+    const int cnt = 1 << (R - 1 - t), off = (1 << (R - 1)) - (1 << (R - t));
+    const uint32_t* src = layer_twiddles(p, t) + (g << (R - 1 - t));
+    if (cnt >= 4) {
+#pragma unroll
+      for (int q = 0; q < cnt; q += 4) {
+        const uint4 x = __ldg(reinterpret_cast<const uint4*>(src + q));
+        w[off + q] = x.x; w[off + q + 1] = x.y; w[off + q + 2] = x.z; w[off + q + 3] = x.w;
+      }
+    } else if (cnt == 2) {
+      const uint2 x = __ldg(reinterpret_cast<const uint2*>(src));
+      w[off] = x.x; w[off + 1] = x.y;
+    } else {
+      w[off] = __ldg(src);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < (1 << (R - 1)) - 1; q++) w[q] <<= 1;
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    const int t = INV ? k : R - 1 - k;
+    if (t > 0) {
+      const int off = (1 << (R - 1)) - (1 << (R - t));
+#pragma unroll
+      for (int j = 0; j < (1 << R); j++) {
+        if (j & (1 << t)) continue;
+        if (INV)
+          ibfly2(v[j], v[j | (1 << t)], w[off + (j >> (t + 1))]);
+        else
+          bfly2(v[j], v[j | (1 << t)], w[off + (j >> (t + 1))]);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < (1 << (R - 1)); q++) {
+        const uint32_t x2 = w[2 * (q >> 2)], y2 = w[2 * (q >> 2) + 1];
+        const uint32_t t2 = (q & 3) < 2 ? y2 : x2;
+        const bool neg = (q & 3) == 1 || (q & 3) == 2;
+        uint32_t &a = v[2 * q], &b = v[2 * q + 1];
+        if (INV) {
+          const uint32_t d = neg ? m31_sub(b, a) : m31_sub(a, b);
+          a = m31_add(a, b);
+          b = mul_doubled(d, t2);
+        } else {
+          const uint32_t m = mul_doubled(b, t2), s = m31_add(a, m), d = m31_sub(a, m);
+          a = neg ? d : s;
+          b = neg ? s : d;
+        }
+      }
+    }
+  }
+}
+
+// x 2^k mod P for a canonic x: a rotation of its 31 bits.
+__device__ __forceinline__ uint32_t mul_pow2(uint32_t x, uint32_t k) { return __funnelshift_l(x << 1, x, k) & P; }
+
+// Register budget: 64 registers for 32 values a thread (1024 threads an SM), 40 for 16 or fewer.
+template <int TB>
+constexpr int direct_min_blocks(int threads) {
+  const int b = (TB >= 6 ? 512 : TB == 5 ? 1024 : 1536) / threads;
+  return b < 24 ? b : 24;
+}
+
+// Shared words of one group of a contiguous pass: four pad words per 32, so that both the row
+// accesses (a thread's 2^TA consecutive words, as 16-byte words) and the column accesses (2^TA
+// consecutive words by as many lanes) are conflict-free; the skew puts neighbouring groups'
+// columns on different banks.
+template <int T>
+__host__ __device__ constexpr uint32_t contig_group_words() {
+  constexpr uint32_t w = (1u << T) + (1u << T) / 8;
+  return T >= 10 ? w : w + (((1u << (T / 2)) + 32 - w % 32) % 32);
+}
+__device__ __forceinline__ constexpr uint32_t contig_pad(uint32_t m) { return m + ((m >> 5) << 2); }
+
+constexpr int kContigWarps = 4;
+
+template <int T>
+constexpr uint32_t contig_warp_words() {
+  constexpr int TA = T / 2, TB = T - TA;
+  return (32u >> TA) * (contig_group_words<T>() + (1u << TB));
+}
+
+// Layers [0, T): a warp owns 32 >> TA whole groups of one column (2^(5 + TB) consecutive words).
+// The block's warps take 2^log_wt neighbouring tiles of kContigWarps >> log_wt columns. Columns
+// shorter than a warp's words are transformed by several lanes alike (indexes wrap).
+template <bool INV, int T>
+__global__ void __launch_bounds__(32 * kContigWarps, direct_min_blocks<T - T / 2>(32 * kContigWarps))
+    fft_contig_kernel(const __grid_constant__ FftBatch batch, const FftPass p, uint32_t n_cols, uint32_t log_wt) {
+  constexpr int TA = T / 2, TB = T - TA, V = 1 << TB, GPW = 32 >> TA;
+  constexpr uint32_t GS = contig_group_words<T>();
+  extern __shared__ __align__(16) uint32_t smem[];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t col = blockIdx.y * (kContigWarps >> log_wt) + (warp >> log_wt);
+  const uint32_t tile = (blockIdx.x << log_wt) + (warp & ((1u << log_wt) - 1));
+  const uint32_t n_mask = (1u << p.log_n) - 1, g_mask = n_mask >> T;
+  if (col >= n_cols || tile * (32u * V) > n_mask) return;
+  uint32_t* s = smem + warp * contig_warp_words<T>();
+  uint32_t* tab = s + GPW * GS;
+  const uint32_t* src = batch.src[col];
+  uint32_t* dst = batch.dst[col];
+  const uint32_t gl = lane >> TA, ml = lane & ((1u << TA) - 1);
+  const uint32_t g = (tile * GPW + gl) & g_mask;
+  uint32_t* sg = s + gl * GS;
+  uint32_t v[V];
+  fill_table<TB>(p, TA, lane, GPW, tab, [&](int k) { return (tile * GPW + k) & g_mask; });
+  if (INV) {
+    if (p.vec) {
+#pragma unroll
+      for (int k = 0; k < V / 4; k++) {
+        const uint32_t L = 4 * lane + 128 * k;
+        const uint4 x = __ldg(reinterpret_cast<const uint4*>(src + ((tile * (32u * V) + L) & n_mask)));
+        *reinterpret_cast<uint4*>(s + (L >> T) * GS + contig_pad(L & ((1u << T) - 1))) = x;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < V; k++) {
+        const uint32_t L = lane + 32 * k;
+        s[(L >> T) * GS + contig_pad(L & ((1u << T) - 1))] = __ldg(src + ((tile * (32u * V) + L) & n_mask));
+      }
+    }
+  } else {
+    const uint32_t* q = src + (((g << T) & p.src_mask) | ml);
+#pragma unroll
+    for (int j = 0; j < V; j++) v[j] = __ldg(q + (j << TA));
+  }
+  __syncwarp();
+  if (!INV) {
+    table_stage<INV, TB>(v, tab + (gl << TB));
+#pragma unroll
+    for (int j = 0; j < V; j++) sg[contig_pad(j << TA) + ml] = v[j];
+    __syncwarp();
+  }
+#pragma unroll
+  for (int r = 0; r < (1 << (TB - TA)); r++) {
+    const uint32_t ma = ml | (r << TA);
+    uint4* row = reinterpret_cast<uint4*>(sg + contig_pad(ma << TA));
+    uint32_t* u = v + (r << TA);
+#pragma unroll
+    for (int q = 0; q < (1 << TA) / 4; q++) {
+      const uint4 x = row[q];
+      u[4 * q] = x.x; u[4 * q + 1] = x.y; u[4 * q + 2] = x.z; u[4 * q + 3] = x.w;
+    }
+    circle_stage<INV, TA>(p, (g << TB) | ma, u);
+#pragma unroll
+    for (int q = 0; q < (1 << TA) / 4; q++) row[q] = make_uint4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+  }
+  __syncwarp();
+  if (INV) {
+#pragma unroll
+    for (int j = 0; j < V; j++) v[j] = sg[contig_pad(j << TA) + ml];
+    table_stage<INV, TB>(v, tab + (gl << TB));
+    uint32_t* q = dst + ((g << T) | ml);
+    if (p.scale) {
+      const uint32_t k = __ffs(p.scale) - 1;
+#pragma unroll
+      for (int j = 0; j < V; j++) v[j] = mul_pow2(v[j], k);
+    }
+#pragma unroll
+    for (int j = 0; j < V; j++) q[j << TA] = v[j];
+  } else if (p.vec) {
+#pragma unroll
+    for (int k = 0; k < V / 4; k++) {
+      const uint32_t L = 4 * lane + 128 * k;
+      *reinterpret_cast<uint4*>(dst + ((tile * (32u * V) + L) & n_mask)) =
+          *reinterpret_cast<const uint4*>(s + (L >> T) * GS + contig_pad(L & ((1u << T) - 1)));
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      const uint32_t L = lane + 32 * k;
+      dst[(tile * (32u * V) + L) & n_mask] = s[(L >> T) * GS + contig_pad(L & ((1u << T) - 1))];
+    }
+  }
+}
+
+// A strided tile holds [m][e] with 8 pad words per stage row (2^TA values of m), so that a warp's
+// four rows fall on distinct banks.
+template <int TA, int EB>
+__device__ __forceinline__ constexpr uint32_t strided_pad(uint32_t L) {
+  return L + ((L >> (TA + EB)) << EB);
+}
+template <int T, int EB>
+constexpr uint32_t strided_tile_words() {
+  return (1u << (EB + T)) + (1u << (EB + T - T / 2));
+}
+template <int T, int EB>
+constexpr uint32_t strided_smem_words() {
+  constexpr int TA = T / 2, TB = T - TA;
+  return strided_tile_words<T, EB>() + (((1u << EB) << TA) / 32) * ((1u << TB) + ((32u >> EB) << TB));
+}
+
+// Layers [lo, lo + T), lo >= 3: a block owns the 2^T values of 8 neighbouring groups (32-byte runs
+// in memory), one (group, stage row) a thread.
+template <bool INV, int T, int EB>
+__global__ void __launch_bounds__((1 << EB) << (T / 2), direct_min_blocks<T - T / 2>((1 << EB) << (T / 2)))
+    fft_strided_kernel(const __grid_constant__ FftBatch batch, const FftPass p) {
+  constexpr int TA = T / 2, TB = T - TA, V = 1 << TB;
+  extern __shared__ __align__(16) uint32_t smem[];
+  const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  constexpr int RW = 32 >> EB;  // rows a warp
+  const uint32_t e = t & ((1u << EB) - 1), ml = t >> EB;
+  uint32_t* tabB = smem + strided_tile_words<T, EB>() + warp * ((1u + RW) << TB);
+  uint32_t* tabA = tabB + (1 << TB);
+  // replicated reads (evaluate's first pass): the replicas of a tile are neighbouring blocks and
+  // share its reads; otherwise neighbouring runs of the same lines are
+  const uint32_t outer_bits = p.log_n - p.hi, run_bits = p.lo - EB;
+  uint32_t o, ib;
+  if (p.src_mask != 0xffffffffu) {
+    o = blockIdx.x & ((1u << outer_bits) - 1);
+    ib = blockIdx.x >> outer_bits;
+  } else {
+    ib = blockIdx.x & ((1u << run_bits) - 1);
+    o = blockIdx.x >> run_bits;
+  }
+  const uint32_t base = (o << p.hi) | (ib << EB) | e;
+  const uint32_t* src = batch.src[blockIdx.y] + (base & p.src_mask);
+  uint32_t* dst = batch.dst[blockIdx.y] + base;
+  // rows 4 warp .. 4 warp + 3 (and the same plus 2^TA) of the low stage are this warp's
+  const uint32_t row0 = (o << TB) | (warp * RW);
+  fill_table<TB>(p, p.lo + TA, lane, 1, tabB, [&](int) { return o; });
+  fill_table<TA>(p, p.lo, lane, RW << (TB - TA), tabA,
+                 [&](int k) { return row0 + (k & (RW - 1)) + ((uint32_t)(k >> (5 - EB)) << TA); });
+  uint32_t v[V];
+  if (INV) {
+#pragma unroll
+    for (int r = 0; r < (1 << (TB - TA)); r++) {
+      const uint32_t* q = src + ((size_t)(ml | (r << TA)) << (p.lo + TA));
+#pragma unroll
+      for (int j = 0; j < (1 << TA); j++) v[(r << TA) + j] = __ldg(q + ((size_t)j << p.lo));
+    }
+  } else {
+    const uint32_t* q = src + ((size_t)ml << p.lo);
+#pragma unroll
+    for (int j = 0; j < V; j++) v[j] = __ldg(q + ((size_t)j << (p.lo + TA)));
+  }
+  __syncwarp();
+#pragma unroll
+  for (int phase = 0; phase < 2; phase++) {
+    const bool low = INV ? phase == 0 : phase == 1;
+    if (phase == 1) __syncthreads();
+    if (low) {
+#pragma unroll
+      for (int r = 0; r < (1 << (TB - TA)); r++) {
+        uint32_t* u = v + (r << TA);
+        uint32_t* row = smem + strided_pad<TA, EB>((((ml | (r << TA)) << TA) << EB) | e);
+        if (!INV) {
+#pragma unroll
+          for (int j = 0; j < (1 << TA); j++) u[j] = row[j << EB];
+        }
+        table_stage<INV, TA>(u, tabA + (((ml & (RW - 1)) | (r << (5 - EB))) << TA));
+        if (INV) {
+#pragma unroll
+          for (int j = 0; j < (1 << TA); j++) row[j << EB] = u[j];
+        }
+      }
+    } else {
+      if (INV) {
+#pragma unroll
+        for (int j = 0; j < V; j++) v[j] = smem[strided_pad<TA, EB>((j << TA) << EB) + ((ml << EB) | e)];
+      }
+      table_stage<INV, TB>(v, tabB);
+      if (!INV) {
+#pragma unroll
+        for (int j = 0; j < V; j++) smem[strided_pad<TA, EB>((j << TA) << EB) + ((ml << EB) | e)] = v[j];
+      }
+    }
+  }
+  if (INV) {
+    if (p.scale) {
+      const uint32_t k = __ffs(p.scale) - 1;
+#pragma unroll
+      for (int j = 0; j < V; j++) v[j] = mul_pow2(v[j], k);
+    }
+    uint32_t* q = dst + ((size_t)ml << p.lo);
+#pragma unroll
+    for (int j = 0; j < V; j++) q[(size_t)j << (p.lo + TA)] = v[j];
+  } else {
+#pragma unroll
+    for (int r = 0; r < (1 << (TB - TA)); r++) {
+      uint32_t* q = dst + ((size_t)(ml | (r << TA)) << (p.lo + TA));
+#pragma unroll
+      for (int j = 0; j < (1 << TA); j++) q[(size_t)j << p.lo] = v[(r << TA) + j];
+    }
+  }
+}
+
 // Domains of log size 1 and 2 use the half coset's first point directly
 // (cpu/circle.rs:34-58 and :203-223). One thread per column.
 struct SmallParams {
@@ -454,6 +819,20 @@ std::map<PlanKey, std::vector<uint32_t>> g_plans;
 
 constexpr uint32_t kMaxContiguousPass = 12, kMaxStridedPass = 11, kStridedC = 3;
 
+// The default split: one pass of up to 12 layers, two passes of up to 22 (a 10-layer first pass for
+// 17-20 layers: the longest with 1024 threads an SM in both), else a 10-layer first pass and two
+// strided ones. Measured (interpolate / evaluate at blowup 1, us): 32 x 2^22 as (11, 11) 640 / 1153,
+// (8, 7, 7) 648 / 1203; 8 x 2^23 as (10, 7, 6) 340 / 621, (12, 11) 393 / 721; 1 x 2^24 as
+// (10, 7, 7) 100 / 178, (8, 8, 8) 103 / 183; 64 x 2^19 as (10, 9) 155 / 263, (11, 8) 164 / 279.
+std::vector<uint32_t> default_split(uint32_t n_layers) {
+  if (n_layers <= kMaxContiguousPass) return {n_layers};
+  if (n_layers <= 2 * kMaxStridedPass) {
+    const uint32_t first = n_layers >= 17 && n_layers <= 20 ? 10 : (n_layers + 1) / 2;
+    return {first, n_layers - first};
+  }
+  return {10, (n_layers - 9) / 2, (n_layers - 10) / 2};
+}
+
 // Splits layers [0, n_layers) of a column of log size log_n into passes of at
 // most 12 layers (11 for strided passes); the first pass is contiguous.
 std::vector<PassPlan> plan_passes(bool inverse, uint32_t log_n, uint32_t n_layers) {
@@ -464,17 +843,7 @@ std::vector<PassPlan> plan_passes(bool inverse, uint32_t log_n, uint32_t n_layer
     auto it = g_plans.find(PlanKey{inverse ? 1u : 0u, log_n, n_layers});
     if (it != g_plans.end()) sizes = it->second;
   }
-  if (sizes.empty()) {
-    uint32_t n_pass = 1;
-    while (n_layers > kMaxContiguousPass + (n_pass - 1) * kMaxStridedPass) n_pass++;
-    sizes.resize(n_pass);
-    const uint32_t base = n_layers / n_pass, extra = n_layers % n_pass;
-    // the contiguous first pass takes the remainder, so strided passes stay <= 11
-    for (uint32_t i = 0; i < n_pass; i++) sizes[i] = base + (i < extra ? 1 : 0);
-    // two passes of 17-20 layers: a 10-layer first pass (tiles of up to 10 layers run four blocks
-    // per SM); measured 7-11% faster than (9, 9) at 18 layers, equal elsewhere in the range
-    if (n_pass == 2 && n_layers >= 17 && n_layers <= 20) sizes = {10, n_layers - 10};
-  }
+  if (sizes.empty()) sizes = default_split(n_layers);
   const uint32_t n_pass = (uint32_t)sizes.size();
   uint32_t lo = 0;
   for (uint32_t i = 0; i < n_pass; i++) {
@@ -522,20 +891,82 @@ cs_status launch_tile(const FftBatch& b, uint32_t n_cols, const FftPass& p, cuda
   return CS_OK;
 }
 
+// Raises a kernel's shared-memory limit once per device (the limit is a per-device attribute of the
+// kernel; several prover threads may launch the first FFT of a device at once).
+template <typename Kernel>
+cs_status allow_smem(Kernel kernel, size_t bytes, std::mutex& mu, bool* configured) {
+  if (bytes <= 48 * 1024) return CS_OK;
+  int dev = 0;
+  CS_CUDA(cudaGetDevice(&dev));
+  CS_CHECK_ARG(dev >= 0 && dev < kMaxDevices, "fft: device ordinal %d out of range", dev);
+  std::lock_guard<std::mutex> lock(mu);
+  if (!configured[dev]) {
+    CS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    configured[dev] = true;
+  }
+  return CS_OK;
+}
+
+template <bool INV, int T>
+cs_status launch_contig(const FftBatch& b, uint32_t n_cols, const FftPass& p, cudaStream_t st) {
+  constexpr size_t smem = sizeof(uint32_t) * kContigWarps * contig_warp_words<T>();
+  static_assert(smem <= 48 * 1024, "contiguous pass: shared memory");
+  // the warps of a block take the same tile of several columns, whose twiddles they share through
+  // L1, and neighbouring tiles where there are too few columns
+  const uint32_t log_wt = n_cols >= 4 ? 0 : n_cols >= 2 ? 1 : 2;
+  constexpr uint32_t log_words = 5 + T - T / 2;
+  const uint32_t log_tiles = p.log_n > log_words ? p.log_n - log_words : 0;
+  dim3 grid(1u << (log_tiles > log_wt ? log_tiles - log_wt : 0),
+            (n_cols + (kContigWarps >> log_wt) - 1) / (kContigWarps >> log_wt));
+  fft_contig_kernel<INV, T><<<grid, 32 * kContigWarps, smem, st>>>(b, p, n_cols, log_wt);
+  CS_LAUNCHED("fft_contig_kernel");
+  return CS_OK;
+}
+
+template <bool INV, int T, int EB>
+cs_status launch_strided_runs(const FftBatch& b, uint32_t n_cols, const FftPass& p, cudaStream_t st) {
+  constexpr size_t smem = sizeof(uint32_t) * strided_smem_words<T, EB>();
+  static std::mutex mu;
+  static bool configured[kMaxDevices] = {false};
+  const cs_status s = allow_smem(fft_strided_kernel<INV, T, EB>, smem, mu, configured);
+  if (s != CS_OK) return s;
+  dim3 grid(1u << (p.log_n - T - EB), n_cols);
+  fft_strided_kernel<INV, T, EB><<<grid, (1 << EB) << (T / 2), smem, st>>>(b, p);
+  CS_LAUNCHED("fft_strided_kernel");
+  return CS_OK;
+}
+
+// 64-byte runs (16 groups a tile) where the block stays at 256 threads or fewer: up to 9 layers,
+// measured 1-4% faster than 32-byte runs on passes of 6-9 layers (256 columns of 2^20 as (7, 7, 6):
+// interpolate 1255 against 1294 us, evaluate onto 2^22 4637 against 4773 us). Passes of 10 and 11
+// layers lose 3-6% to the wider block's barrier (256 x 2^20 as (10, 10): evaluate 3811 against
+// 3690 us) and keep 8 groups.
+template <bool INV, int T>
+cs_status launch_strided(const FftBatch& b, uint32_t n_cols, const FftPass& p, cudaStream_t st) {
+  if constexpr (T <= 9) {
+    if (p.lo >= 4) return launch_strided_runs<INV, T, 4>(b, n_cols, p, st);
+  }
+  return launch_strided_runs<INV, T, 3>(b, n_cols, p, st);
+}
+
 template <bool INV, bool OUTER>
 cs_status dispatch_tile(const FftBatch& b, uint32_t n_cols, const FftPass& p, cudaStream_t st) {
   switch (p.hi - p.lo) {
     case 1: return launch_tile<INV, 1, OUTER>(b, n_cols, p, st);
     case 2: return launch_tile<INV, 2, OUTER>(b, n_cols, p, st);
     case 3: return launch_tile<INV, 3, OUTER>(b, n_cols, p, st);
-    case 4: return launch_tile<INV, 4, OUTER>(b, n_cols, p, st);
-    case 5: return launch_tile<INV, 5, OUTER>(b, n_cols, p, st);
-    case 6: return launch_tile<INV, 6, OUTER>(b, n_cols, p, st);
-    case 7: return launch_tile<INV, 7, OUTER>(b, n_cols, p, st);
-    case 8: return launch_tile<INV, 8, OUTER>(b, n_cols, p, st);
-    case 9: return launch_tile<INV, 9, OUTER>(b, n_cols, p, st);
-    case 10: return launch_tile<INV, 10, OUTER>(b, n_cols, p, st);
-    case 11: return launch_tile<INV, 11, OUTER>(b, n_cols, p, st);
+    case 4:
+      if constexpr (!OUTER) return launch_strided<INV, 4>(b, n_cols, p, st);
+      else return launch_tile<INV, 4, OUTER>(b, n_cols, p, st);
+    case 5:
+      if constexpr (!OUTER) return launch_strided<INV, 5>(b, n_cols, p, st);
+      else return launch_tile<INV, 5, OUTER>(b, n_cols, p, st);
+    case 6: return OUTER ? launch_contig<INV, 6>(b, n_cols, p, st) : launch_strided<INV, 6>(b, n_cols, p, st);
+    case 7: return OUTER ? launch_contig<INV, 7>(b, n_cols, p, st) : launch_strided<INV, 7>(b, n_cols, p, st);
+    case 8: return OUTER ? launch_contig<INV, 8>(b, n_cols, p, st) : launch_strided<INV, 8>(b, n_cols, p, st);
+    case 9: return OUTER ? launch_contig<INV, 9>(b, n_cols, p, st) : launch_strided<INV, 9>(b, n_cols, p, st);
+    case 10: return OUTER ? launch_contig<INV, 10>(b, n_cols, p, st) : launch_strided<INV, 10>(b, n_cols, p, st);
+    case 11: return OUTER ? launch_contig<INV, 11>(b, n_cols, p, st) : launch_strided<INV, 11>(b, n_cols, p, st);
     case 12:
       // plan_passes keeps strided passes at 11 layers or fewer
       if constexpr (OUTER) return launch_tile<INV, 12, OUTER>(b, n_cols, p, st);
