@@ -50,19 +50,46 @@ inline uint32_t fma_add(uint32_t a, uint32_t one, uint32_t b) { return a * one +
   c = fma_add(c, one, d);          \
   b = rotr7(b ^ c);
 
+// The same step for a chain of dependent compressions on few warps, where the latency of a step
+// counts and not the ALU pipe's rate: all additions as they are. One warp alone takes 1,672 cycles
+// a compression this way against 3,155 with the multiply-adds; from about 256 threads an SM on the
+// multiply-adds are the faster form (1024 threads: 11,351 against 13,077).
+#define CS_B2S_G_CHAIN(a, b, c, d, x, y) \
+  a = a + b + (x);                       \
+  d = rotr16(d ^ a);                     \
+  c = c + d;                             \
+  b = rotr12(b ^ c);                     \
+  a = a + b + (y);                       \
+  d = rotr8(d ^ a);                      \
+  c = c + d;                             \
+  b = rotr7(b ^ c);
+
 #define CS_B2S_ROUND(s0, s1, s2, s3, s4, s5, s6, s7, s8, s9, s10, s11, s12, s13, s14, s15) \
-  CS_B2S_G(v0, v4, v8, v12, m[s0], m[s1])                                                   \
-  CS_B2S_G(v1, v5, v9, v13, m[s2], m[s3])                                                   \
-  CS_B2S_G(v2, v6, v10, v14, m[s4], m[s5])                                                  \
-  CS_B2S_G(v3, v7, v11, v15, m[s6], m[s7])                                                  \
-  CS_B2S_G(v0, v5, v10, v15, m[s8], m[s9])                                                  \
-  CS_B2S_G(v1, v6, v11, v12, m[s10], m[s11])                                                \
-  CS_B2S_G(v2, v7, v8, v13, m[s12], m[s13])                                                 \
-  CS_B2S_G(v3, v4, v9, v14, m[s14], m[s15])
+  if (CHAIN) {                                                                              \
+    CS_B2S_G_CHAIN(v0, v4, v8, v12, m[s0], m[s1])                                           \
+    CS_B2S_G_CHAIN(v1, v5, v9, v13, m[s2], m[s3])                                           \
+    CS_B2S_G_CHAIN(v2, v6, v10, v14, m[s4], m[s5])                                          \
+    CS_B2S_G_CHAIN(v3, v7, v11, v15, m[s6], m[s7])                                          \
+    CS_B2S_G_CHAIN(v0, v5, v10, v15, m[s8], m[s9])                                          \
+    CS_B2S_G_CHAIN(v1, v6, v11, v12, m[s10], m[s11])                                        \
+    CS_B2S_G_CHAIN(v2, v7, v8, v13, m[s12], m[s13])                                         \
+    CS_B2S_G_CHAIN(v3, v4, v9, v14, m[s14], m[s15])                                         \
+  } else {                                                                                  \
+    CS_B2S_G(v0, v4, v8, v12, m[s0], m[s1])                                                 \
+    CS_B2S_G(v1, v5, v9, v13, m[s2], m[s3])                                                 \
+    CS_B2S_G(v2, v6, v10, v14, m[s4], m[s5])                                                \
+    CS_B2S_G(v3, v7, v11, v15, m[s6], m[s7])                                                \
+    CS_B2S_G(v0, v5, v10, v15, m[s8], m[s9])                                                \
+    CS_B2S_G(v1, v6, v11, v12, m[s10], m[s11])                                              \
+    CS_B2S_G(v2, v7, v8, v13, m[s12], m[s13])                                               \
+    CS_B2S_G(v3, v4, v9, v14, m[s14], m[s15])                                               \
+  }
 
 // h: chaining value (in/out). m: 16 message words. t: byte counter after this
 // block. last: whether this is the final block. one: the value 1, passed in at
 // run time (a kernel parameter) so the additions above stay multiply-adds.
+// CHAIN: the low-latency form, for kernels that run few compressions at a time.
+template <bool CHAIN = false>
 __host__ __device__ __forceinline__ void b2s_compress(uint32_t h[8], const uint32_t m[16], uint32_t t_lo,
                                                       uint32_t t_hi, bool last, uint32_t one = 1) {
   uint32_t v0 = h[0], v1 = h[1], v2 = h[2], v3 = h[3], v4 = h[4], v5 = h[5], v6 = h[6], v7 = h[7];

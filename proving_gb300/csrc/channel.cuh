@@ -55,7 +55,7 @@ __device__ __forceinline__ void channel_mix_root(uint32_t state[9], const uint32
   uint32_t m[16], h[8];
   channel_mix_message(state, root, m);
   b2s_init(h);
-  b2s_compress(h, m, kChannelMixBytes, 0, true);
+  b2s_compress<true>(h, m, kChannelMixBytes, 0, true);
   channel_after_mix(state, h);
 }
 
@@ -63,7 +63,7 @@ __device__ __forceinline__ void channel_draw_felt(uint32_t state[9], uint32_t fe
   uint32_t m[16], h[8];
   channel_draw_message(state, m);
   b2s_init(h);
-  b2s_compress(h, m, kChannelDrawBytes, 0, true);
+  b2s_compress<true>(h, m, kChannelDrawBytes, 0, true);
   channel_after_draw(state, h, felt);
 }
 

@@ -539,9 +539,11 @@ __global__ void __launch_bounds__(kFriTailThreads) fri_tail_kernel(const __grid_
                                                                    uint32_t log_size, uint32_t n_layers,
                                                                    uint32_t* state, uint32_t* alphas,
                                                                    const uint32_t* __restrict__ itw,
-                                                                   uint32_t twiddle_log_size, uint32_t one) {
+                                                                   uint32_t twiddle_log_size) {
   __shared__ uint32_t v[4][1u << kFriTailMaxLog];  // the layer being committed and folded
-  __shared__ uint32_t d[kFriTailThreads][8];       // the tree level being built
+  // the tree level being built, word by word: a node's message is one 8-byte read per word, free of
+  // bank conflicts
+  __shared__ __align__(8) uint32_t d[8][kFriTailThreads];
   __shared__ uint32_t chan[9];
   __shared__ uint32_t alpha[4];
   const uint32_t t = threadIdx.x;
@@ -581,12 +583,21 @@ __global__ void __launch_bounds__(kFriTailThreads) fri_tail_kernel(const __grid_
         on = t < (1u << level);
         if (on) {
 #pragma unroll
-          for (int w = 0; w < 8; w++) msg[w] = d[2 * t][w], msg[8 + w] = d[2 * t + 1][w];
+          for (int w = 0; w < 8; w++) {
+            const uint2 x = *reinterpret_cast<const uint2*>(&d[w][2 * t]);
+            msg[w] = x.x;
+            msg[8 + w] = x.y;
+          }
         }
-      } else if (step == n_steps - 2) {  // mix the root (d[0]) into the channel
+      } else if (step == n_steps - 2) {  // mix the root (node 0) into the channel
         on = t == 0;
         tlo = kChannelMixBytes;
-        if (on) channel_mix_message(chan, d[0], msg);
+        if (on) {
+          uint32_t root[8];
+#pragma unroll
+          for (int w = 0; w < 8; w++) root[w] = d[w][0];
+          channel_mix_message(chan, root, msg);
+        }
       } else {  // draw the folding challenge
         on = t == 0;
         tlo = kChannelDrawBytes;
@@ -595,7 +606,7 @@ __global__ void __launch_bounds__(kFriTailThreads) fri_tail_kernel(const __grid_
       uint32_t h[8];
       if (on) {
         b2s_init(h);
-        b2s_compress(h, msg, tlo, 0, true, one);
+        b2s_compress<true>(h, msg, tlo, 0, true);
       }
       if (step < 2) {
         if (on) {
@@ -612,7 +623,7 @@ __global__ void __launch_bounds__(kFriTailThreads) fri_tail_kernel(const __grid_
         __syncthreads();  // every read of this level's children is done
         if (on) {
 #pragma unroll
-          for (int w = 0; w < 8; w++) d[t][w] = h[w];
+          for (int w = 0; w < 8; w++) d[w][t] = h[w];
           store_digest(tree + ((size_t)(2u << m) - (2u << level) + t) * 8, h);
         }
         __syncthreads();
@@ -922,7 +933,7 @@ extern "C" cs_status cs_fri_commit_fold_tail(uint32_t* d_state, uint32_t* d_alph
   }
   const uint32_t threads = std::max(32u, 1u << (log_size - 1));
   fri_tail_kernel<<<1, threads, 0, to_stream(stream)>>>(T, log_size, n_layers, d_state, d_alphas, d_itwiddles,
-                                                        twiddle_log_size, 1u);
+                                                        twiddle_log_size);
   CS_LAUNCHED("fri_tail_kernel");
   return CS_OK;
 }

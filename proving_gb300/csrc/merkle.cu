@@ -29,6 +29,7 @@ namespace {
 
 constexpr uint32_t kMaxLeafCols = 2048;
 constexpr int kLeafThreads = 128;
+constexpr uint32_t kChainLeaves = 256 * 152;  // up to 256 threads an SM the low-latency compression is faster
 
 struct LeafParams {
   const uint32_t* cols[kMaxLeafCols];
@@ -47,6 +48,10 @@ __device__ __forceinline__ uint32_t lift_index(uint32_t x, uint32_t from, uint32
   return from == to ? x : (((x >> (from - to + 1)) << 1) | (x & 1));
 }
 
+// LIFTED: some column is shorter than the launch's size (an index per column; otherwise every column
+// is read at x, which takes a tenth of the kernel's instructions off). CHAIN: the compression's
+// low-latency form, for launches of few warps an SM.
+template <bool LIFTED, bool CHAIN>
 __global__ void __launch_bounds__(kLeafThreads) merkle_leaves_kernel(const __grid_constant__ LeafParams p,
                                                                      uint32_t* __restrict__ out) {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -57,7 +62,7 @@ __global__ void __launch_bounds__(kLeafThreads) merkle_leaves_kernel(const __gri
     b2s_init(h);
 #pragma unroll
     for (int k = 0; k < 16; k++) m[k] = 0;
-    b2s_compress(h, m, 0, 0, true);
+    b2s_compress<true>(h, m, 0, 0, true);
   } else {
     if (p.prev_state != nullptr) {
       const uint4* src = reinterpret_cast<const uint4*>(p.prev_state + (size_t)lift_index(x, p.level_log, p.prev_log) * 8);
@@ -76,11 +81,11 @@ __global__ void __launch_bounds__(kLeafThreads) merkle_leaves_kernel(const __gri
         uint32_t v = 0;
         if ((uint32_t)k < cnt) {
           const uint32_t c = base + k;
-          v = __ldg(p.cols[c] + lift_index(x, p.level_log, p.log[c]));
+          v = __ldg(p.cols[c] + (LIFTED ? lift_index(x, p.level_log, p.log[c]) : x));
         }
         m[k] = v;
       }
-      b2s_compress(h, m, (base + cnt) * 4, 0, last, p.one);
+      b2s_compress<CHAIN>(h, m, (base + cnt) * 4, 0, last, p.one);
     }
   }
   uint4* o = reinterpret_cast<uint4*>(out + (size_t)x * 8);
@@ -110,37 +115,66 @@ __global__ void merkle_node_kernel(const uint32_t* __restrict__ prev, uint32_t l
   o[1] = make_uint4(h[4], h[5], h[6], h[7]);
 }
 
-// The top layers of a tree in one launch: one block builds layers log_in - 1 down to 0 from the
-// layer of 2^log_in digests at `layer`, each written right after the one before it (the layout of
-// cs_merkle_commit), with a barrier between layers. Plain loads, since each layer reads what the
-// block wrote for the previous one; the barrier makes those stores visible to the block.
-constexpr uint32_t kTopLayersLog = 10;  // layers of up to 2^10 nodes
+// S node layers in one launch: block b builds the subtree over digests [b << S, (b + 1) << S) of the
+// layer of 2^log_in digests at `layer`, every level also written to its layer (the layout of
+// cs_merkle_commit: layers follow one another, leaves first). The level being read and the one being
+// written are in shared memory word by word (a node's message is one 8-byte read per word, and its
+// digest a word store per word, both free of bank conflicts); from 32 nodes on one warp goes on alone.
+// Bound: with few blocks the chain of S compressions (0.8 us each, see b2s_compress), which a launch
+// per layer stretched by a launch's latency and two trips through L2 per layer; with many blocks the
+// ALU pipe, of which the short upper levels use a part only: 35 warp compressions for the 32 that the
+// nodes of S = 10 need, 12 for 8 with S = 8.
+constexpr uint32_t kSubtreeMaxLog = 10;
 
-__global__ void __launch_bounds__(1024) merkle_top_kernel(uint32_t* layer, uint32_t log_in, uint32_t one) {
-  const uint32_t* prev = layer;
-  uint32_t* out = layer + ((size_t)8 << log_in);
-  for (int k = (int)log_in - 1; k >= 0; k--) {
-    for (uint32_t i = threadIdx.x; i < (1u << k); i += blockDim.x) {
-      const uint4* src = reinterpret_cast<const uint4*>(prev + (size_t)i * 16);
-      uint32_t m[16];
+template <bool CHAIN>
+__global__ void __launch_bounds__(256) merkle_subtree_kernel(uint32_t* layer, uint32_t log_in, uint32_t S,
+                                                             uint32_t one) {
+  __shared__ __align__(8) uint32_t even[8][1u << (kSubtreeMaxLog - 1)];  // levels 1, 3, ...
+  __shared__ __align__(8) uint32_t odd[8][1u << (kSubtreeMaxLog - 2)];   // levels 2, 4, ...
+  for (uint32_t k = 1; k <= S; k++) {
+    const uint32_t n = 1u << (S - k);
+    // layer of log size log_in - k: after 2^log_in + ... + 2^(log_in - k + 1) digests
+    uint32_t* out = layer + 8 * (((size_t)2 << log_in) - ((size_t)2 << (log_in - k)) + ((size_t)blockIdx.x << (S - k)));
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+      uint32_t m[16], h[8];
+      if (k == 1) {
+        const uint4* src = reinterpret_cast<const uint4*>(layer + 8 * (((size_t)blockIdx.x << S) + 2 * i));
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint4 w = src[q];
-        m[4 * q] = w.x;
-        m[4 * q + 1] = w.y;
-        m[4 * q + 2] = w.z;
-        m[4 * q + 3] = w.w;
+        for (int q = 0; q < 4; q++) {
+          const uint4 w = src[q];
+          m[4 * q] = w.x;
+          m[4 * q + 1] = w.y;
+          m[4 * q + 2] = w.z;
+          m[4 * q + 3] = w.w;
+        }
+      } else {
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+          const uint2 x = k & 1 ? *reinterpret_cast<const uint2*>(&odd[w][2 * i])
+                                : *reinterpret_cast<const uint2*>(&even[w][2 * i]);
+          m[w] = x.x;
+          m[8 + w] = x.y;
+        }
       }
-      uint32_t h[8];
       b2s_init(h);
-      b2s_compress(h, m, 64, 0, true, one);
-      uint4* o = reinterpret_cast<uint4*>(out + (size_t)i * 8);
+      b2s_compress<CHAIN>(h, m, 64, 0, true, one);
+#pragma unroll
+      for (int w = 0; w < 8; w++) {
+        if (k & 1)
+          even[w][i] = h[w];
+        else
+          odd[w][i] = h[w];
+      }
+      uint4* o = reinterpret_cast<uint4*>(out + 8 * (size_t)i);
       o[0] = make_uint4(h[0], h[1], h[2], h[3]);
       o[1] = make_uint4(h[4], h[5], h[6], h[7]);
     }
-    __syncthreads();
-    prev = out;
-    out += (size_t)8 << k;
+    if (n > 32) {
+      __syncthreads();
+    } else {
+      if (threadIdx.x >= 32) return;
+      __syncwarp();
+    }
   }
 }
 
@@ -203,7 +237,12 @@ cs_status merkle_leaves(const uint32_t* const* cols, const uint32_t* log_sizes, 
     p.prev_log = prev_log;
     uint32_t* dst = top ? d_leaves : states + (r & 1) * half;
     const uint32_t n = 1u << p.level_log;
-    merkle_leaves_kernel<<<(n + kLeafThreads - 1) / kLeafThreads, kLeafThreads, 0, st>>>(p, dst);
+    // the columns are sorted, so the first one tells whether any is shorter than the launch's size
+    const bool lifted = n_cols > 0 && log_sizes[16 * p.block0] != p.level_log;
+    const bool chain = n <= kChainLeaves;
+    auto* kernel = lifted ? (chain ? merkle_leaves_kernel<true, true> : merkle_leaves_kernel<true, false>)
+                          : (chain ? merkle_leaves_kernel<false, true> : merkle_leaves_kernel<false, false>);
+    kernel<<<(n + kLeafThreads - 1) / kLeafThreads, kLeafThreads, 0, st>>>(p, dst);
     note_launch();
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) result = from_cuda(e, "merkle_leaves_kernel");
@@ -229,21 +268,31 @@ cs_status merkle_next_layer(const uint32_t* d_prev, uint32_t log_out, uint32_t* 
   return CS_OK;
 }
 
+// Levels built by the next launch over 2^k digests. Measured (all layers of a tree of height h,
+// CUDA events around the call, of which about 10 us are the measurement's own; before: a launch per
+// layer down to 2^10 nodes, then one block): h = 10: 24.8 -> 22.8 us, h = 12: 34.8 -> 25.7,
+// h = 15: 48.3 -> 29.1, h = 17: 60.2 -> 35.9, h = 20: 108 -> 88, h = 22: 241 -> 225. Below 17 eight
+// levels a launch (ten: 33.1 us at h = 15), since the chain counts and eight start with one node a
+// thread; from 17 on ten (eight: 42.3 us at h = 17, 301 at 22), since the blocks fill the chip and
+// the short upper levels are work for few of their warps.
+uint32_t subtree_levels(uint32_t k) { return k <= 9 ? k : k < 17 ? 8 : kSubtreeMaxLog; }
+
 // Every node layer above the 2^L leaves at d_layers, each right after the one before (leaves
-// first, root last): one launch per layer of more than 2^10 nodes, then the rest in one.
+// first, root last).
 cs_status merkle_layers(uint32_t* d_layers, uint32_t L, cudaStream_t st) {
   uint32_t* cur = d_layers;
-  for (uint32_t k = L; k >= 1; k--) {
-    if (k - 1 <= kTopLayersLog) {
-      const uint32_t threads = std::max(32u, std::min(1024u, 1u << (k - 1)));
-      merkle_top_kernel<<<1, threads, 0, st>>>(cur, k, 1u);
-      CS_LAUNCHED("merkle_top_kernel");
-      break;
-    }
-    uint32_t* next = cur + ((size_t)8 << k);
-    const cs_status s = merkle_next_layer(cur, k - 1, next, st);
-    if (s != CS_OK) return s;
-    cur = next;
+  for (uint32_t k = L; k >= 1;) {
+    const uint32_t S = subtree_levels(k);
+    const uint32_t threads = std::max(32u, std::min(256u, 1u << (S - 1)));
+    const uint32_t blocks = 1u << (k - S);
+    // two blocks an SM or more: the compression's throughput form
+    if (blocks > 2 * 152)
+      merkle_subtree_kernel<false><<<blocks, threads, 0, st>>>(cur, k, S, 1u);
+    else
+      merkle_subtree_kernel<true><<<blocks, threads, 0, st>>>(cur, k, S, 1u);
+    CS_LAUNCHED("merkle_subtree_kernel");
+    cur += 8 * (((size_t)2 << k) - ((size_t)2 << (k - S)));
+    k -= S;
   }
   return CS_OK;
 }
