@@ -12,38 +12,10 @@
 
 #include "common.cuh"
 #include "field.cuh"
+#include "gkr.cuh"
 
 namespace cs {
 namespace {
-
-struct QIn {
-  const uint32_t* c[4];
-};
-struct QOut {
-  uint32_t* c[4];
-};
-
-__device__ __forceinline__ qm31 q_one() { return qm31_make(1, 0, 0, 0); }
-__device__ __forceinline__ qm31 q_zero() { return qm31_make(0, 0, 0, 0); }
-__device__ __forceinline__ qm31 q_double(qm31 x) { return qm31_add(x, x); }
-
-__device__ __forceinline__ qm31 q_load(const QIn& s, uint32_t i) {
-  return qm31_make(s.c[0][i], s.c[1][i], s.c[2][i], s.c[3][i]);
-}
-__device__ __forceinline__ void q_store(const QOut& d, uint32_t i, qm31 v) {
-  d.c[0][i] = v.a.a;
-  d.c[1][i] = v.a.b;
-  d.c[2][i] = v.b.a;
-  d.c[3][i] = v.b.b;
-}
-// values 2i and 2i + 1 of a secure column (8-byte loads: 2i is even)
-__device__ __forceinline__ void q_load_pair(const QIn& s, uint32_t i, qm31& a, qm31& b) {
-  uint2 w[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) w[k] = reinterpret_cast<const uint2*>(s.c[k])[i];
-  a = qm31_make(w[0].x, w[1].x, w[2].x, w[3].x);
-  b = qm31_make(w[0].y, w[1].y, w[2].y, w[3].y);
-}
 
 __device__ __forceinline__ uint32_t grid_stride() { return gridDim.x * blockDim.x; }
 __device__ __forceinline__ uint32_t global_thread() { return blockIdx.x * blockDim.x + threadIdx.x; }
@@ -55,53 +27,14 @@ uint32_t stream_blocks(uint64_t n, uint32_t threads, uint32_t per_sm) {
 
 // ------------------------------------------------------------ gen_eq_evals
 
-constexpr uint32_t kEqLowBits = 10;    // index bits of the per-block table
-constexpr uint32_t kEqChunkBits = 14;  // values written per block
-constexpr uint32_t kEqMaxVars = 28;
-
 struct EqParams {
   qm31 v;
   qm31 y[kEqMaxVars];
   uint32_t n;
 };
 
-// evals[i] = v * prod_j eq(x_j, y_j), x_j = bit n-1-j of i (gen_eq_evals,
-// cpu/lookups/gkr.rs:230-246: the loop over y in reverse doubles the table, so
-// y[n-1] is index bit 0). Each block builds the factor of the low kEqLowBits
-// bits as a table in shared memory by the same doubling, the factor of its own
-// high bits directly, and writes their products.
-__global__ void __launch_bounds__(256) eq_evals_kernel(const EqParams p, const QOut out) {
-  __shared__ qm31 low[1u << kEqLowBits];
-  __shared__ qm31 high[1u << (kEqChunkBits - kEqLowBits)];
-  const uint32_t n = p.n;
-  const uint32_t k = min(n, kEqLowBits);
-  const uint32_t chunk = min(n, kEqChunkBits);
-  if (threadIdx.x == 0) low[0] = q_one();
-  __syncthreads();
-  for (uint32_t t = 0; t < k; t++) {
-    const qm31 yt = p.y[n - 1 - t];
-    for (uint32_t j = threadIdx.x; j < (1u << t); j += blockDim.x) {
-      const qm31 lj = low[j];
-      const qm31 tmp = qm31_mul(lj, yt);
-      low[j + (1u << t)] = tmp;
-      low[j] = qm31_sub(lj, tmp);
-    }
-    __syncthreads();
-  }
-  const uint32_t first = blockIdx.x << chunk;
-  if (threadIdx.x < (1u << (chunk - k))) {
-    const uint32_t hi = (first >> k) + threadIdx.x;
-    qm31 h = p.v;
-    for (uint32_t t = k; t < n; t++) {
-      const qm31 yt = p.y[n - 1 - t];
-      h = qm31_mul(h, ((hi >> (t - k)) & 1u) ? yt : qm31_sub(q_one(), yt));
-    }
-    high[threadIdx.x] = h;
-  }
-  __syncthreads();
-  const uint32_t low_mask = (1u << k) - 1;
-  for (uint32_t e = threadIdx.x; e < (1u << chunk); e += blockDim.x)
-    q_store(out, first + e, qm31_mul(high[e >> k], low[e & low_mask]));
+__global__ void __launch_bounds__(256) eq_evals_kernel(const __grid_constant__ EqParams p, const QOut out) {
+  eq_evals_block(p.v, p.y, p.n, out);
 }
 
 // ------------------------------------------------------------ fix_first_variable
@@ -163,13 +96,6 @@ __global__ void __launch_bounds__(256) next_layer_kernel(const QIn num, const QI
 }
 
 // ------------------------------------------------------------ sum_as_poly_in_first_variable
-
-__device__ __forceinline__ qm31 q_shfl_add(qm31 v, int off) {
-  return qm31_make(m31_add(v.a.a, __shfl_xor_sync(0xffffffffu, v.a.a, off)),
-                   m31_add(v.a.b, __shfl_xor_sync(0xffffffffu, v.a.b, off)),
-                   m31_add(v.b.a, __shfl_xor_sync(0xffffffffu, v.b.a, off)),
-                   m31_add(v.b.b, __shfl_xor_sync(0xffffffffu, v.b.b, off)));
-}
 
 // Sum of two QM31 values over a 256-thread block; thread 0 gets the totals.
 __device__ __forceinline__ void block_sum2(qm31& s0, qm31& s2) {
