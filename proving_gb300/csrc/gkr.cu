@@ -34,7 +34,7 @@ struct EqParams {
 };
 
 __global__ void __launch_bounds__(256) eq_evals_kernel(const __grid_constant__ EqParams p, const QOut out) {
-  eq_evals_block(p.v, p.y, p.n, out);
+  eq_evals_block(blockIdx.x, p.v, p.y, p.n, out);
 }
 
 // ------------------------------------------------------------ fix_first_variable

@@ -65,7 +65,7 @@ constexpr uint32_t kEqMaxVars = 28;
 // y[n-1] is index bit 0). Each block builds the factor of the low kEqLowBits
 // bits as a table in shared memory by the same doubling, the factor of its own
 // high bits directly, and writes their products.
-__device__ __forceinline__ void eq_evals_block(const qm31 v, const qm31* y, uint32_t n, const QOut& out) {
+__device__ __forceinline__ void eq_evals_block(uint32_t block, const qm31 v, const qm31* y, uint32_t n, const QOut& out) {
   __shared__ qm31 low[1u << kEqLowBits];
   __shared__ qm31 high[1u << (kEqChunkBits - kEqLowBits)];
   const uint32_t k = min(n, kEqLowBits);
@@ -82,7 +82,7 @@ __device__ __forceinline__ void eq_evals_block(const qm31 v, const qm31* y, uint
     }
     __syncthreads();
   }
-  const uint32_t first = blockIdx.x << chunk;
+  const uint32_t first = block << chunk;
   if (threadIdx.x < (1u << (chunk - k))) {
     const uint32_t hi = (first >> k) + threadIdx.x;
     qm31 h = v;

@@ -5,19 +5,22 @@
 //
 // Before, the host ran the protocol over the kernels of gkr.cu: about five launches, their
 // allocations and a synchronising read-back per sum-check round, 60 us a round whatever its size
-// (14.4 ms for the 231 rounds of 2^22 fractions beside 2^20 products). A round's own chain is short:
-// fix, sums, one product per coefficient, three dependent Blake2s compressions. Here a round of many
+// (14.4 ms for the 231 rounds of 2^22 fractions beside 2^20 products; now 3.7). A round's own chain is
+// short: fix, sums, one product per coefficient, three dependent Blake2s compressions. Here a round of many
 // terms is one launch: it fixes the previous variable, writes the halved columns, sums the next
 // round's terms from the same registers, and the last block to finish turns the sums into the round
 // polynomial, mixes it and draws the next challenge. The last kTailRounds rounds of a layer, the
 // layer's masks and the next layer's claims and constants (and whole layers while they are that
-// small) are one single-block launch.
+// small) are one single-block launch. The launches of one proof are a chain of programmatic dependent
+// launches.
 //
-// Bound: latency. A QM31 product is 210 cycles for a lone warp and a compression about 1,800, so the
-// block spreads a round's products over its threads in as few levels as they need: one product per
+// Bound: latency (7.3 us a round in the single-block kernel, 13 in a launch of its own: 4.6 for the
+// terms, 1.5 for the blocks' sums, 4.7 to end the round, 0.7 to the next launch). A QM31 product is
+// 155-220 cycles for a lone warp and a compression about 1,900, so the block spreads a round's products over its threads in as few levels as they need: one product per
 // element to fix, two per part of a term, one per (coefficient, sum), and what only the next round
 // needs (claims, corrections, coefficient tables) runs in other warps beside the next fix.
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -31,8 +34,11 @@
 namespace cs {
 namespace {
 
-// Rounds of up to 2^(kTailRounds - 1) terms run in the single-block kernel.
-constexpr uint32_t kTailRounds = 9;
+// Rounds of up to 2^(kTailRounds - 1) terms run in the single-block kernel: 64 terms are 1,024 items of
+// two products for its 512 threads, about 8 us a round; at 128 and 256 terms a round there takes 15 and
+// 25 us and a launch over several blocks 13 (2^22 + 2^20 with a limit of 6, 7, 8 rounds: 3.78, 3.75,
+// 3.75 ms; 9 before the launches overlapped: 4.30).
+constexpr uint32_t kTailRounds = 7;
 constexpr uint32_t kTailThreads = 512;
 constexpr uint32_t kTailTerms = 1u << (kTailRounds - 1);
 constexpr uint32_t kRoundThreads = 128;
@@ -51,7 +57,7 @@ struct LayerCols {
 };
 
 // The round polynomial is linear in the sums f0, f2 at t = 0, 2 and the claim:
-// coefficient t = corr f0 u[k][t] + corr f2 v[k][t] + claim w[k][t], k variables left
+// coefficient t = corr f0 u[t] + corr f2 v[t] + claim w[t] with the row of the k variables left
 // (correct_sum_as_poly_in_first_variable; RoundConstants of proving_gb300/gkr.py).
 struct GkrState {
   uint32_t chan[9];
@@ -59,7 +65,9 @@ struct GkrState {
   uint32_t pad[6];
   qm31 lam, alpha, x;
   qm31 y[kMaxVars], sc[kMaxVars];  // the point of the layer's claims, this sum-check's challenges
-  qm31 u[kMaxVars][4], v[kMaxVars][4], w[kMaxVars][4];
+  struct {
+    qm31 u[4], v[4], w[4];
+  } row[kMaxVars];  // k variables left
 };
 
 struct InstState {
@@ -94,57 +102,58 @@ __device__ __forceinline__ bool q_is_zero(qm31 v) { return (v.a.a | v.a.b | v.b.
 
 // ------------------------------------------------------------ channel (one warp)
 
-__constant__ uint8_t kSigma[160] = {
-    0,  1,  2,  3,  4,  5,  6,  7,  8,  9,  10, 11, 12, 13, 14, 15, 14, 10, 4,  8,  9,  15, 13, 6,  1,  12, 0,
-    2,  11, 7,  5,  3,  11, 8,  12, 0,  5,  2,  15, 13, 10, 14, 3,  6,  7,  1,  9,  4,  7,  9,  3,  1,  13, 12,
-    11, 14, 2,  6,  5,  10, 4,  0,  15, 8,  9,  0,  5,  7,  2,  4,  10, 15, 14, 1,  11, 12, 6,  8,  3,  13, 2,
-    12, 6,  10, 0,  11, 8,  3,  4,  13, 7,  5,  15, 14, 1,  9,  12, 5,  1,  15, 14, 13, 4,  10, 0,  7,  6,  3,
-    9,  2,  8,  11, 13, 11, 7,  14, 12, 1,  3,  9,  5,  0,  15, 4,  8,  6,  2,  10, 6,  15, 14, 9,  11, 3,  0,
-    8,  12, 2,  13, 7,  1,  4,  10, 5,  10, 2,  8,  4,  7,  6,  1,  5,  15, 11, 9,  14, 3,  12, 13, 0};
+// SIGMA (RFC 7693 section 2.7) by round and lane: the two words of lane q's column step, then those of
+// its diagonal step.
+__device__ const uint8_t kSigma[160] = {
+    0, 1, 8, 9, 2, 3, 10, 11, 4, 5, 12, 13, 6, 7, 14, 15, 14, 10, 1, 12, 4, 8, 0, 2, 9, 15, 11, 7, 13, 6, 5, 3,
+    11, 8, 10, 14, 12, 0, 3, 6, 5, 2, 7, 1, 15, 13, 9, 4, 7, 9, 2, 6, 3, 1, 5, 10, 13, 12, 4, 0, 11, 14, 15, 8,
+    9, 0, 14, 1, 5, 7, 11, 12, 2, 4, 6, 8, 10, 15, 3, 13, 2, 12, 4, 13, 6, 10, 7, 5, 0, 11, 15, 14, 8, 3, 1, 9,
+    12, 5, 0, 7, 1, 15, 6, 3, 14, 13, 9, 2, 4, 10, 8, 11, 13, 11, 5, 0, 7, 14, 15, 4, 12, 1, 8, 6, 3, 9, 2, 10,
+    6, 15, 12, 2, 14, 9, 13, 7, 11, 3, 1, 4, 0, 8, 10, 5, 10, 2, 15, 11, 8, 4, 9, 14, 7, 6, 3, 12, 1, 5, 13, 0};
 
 struct Hash {
-  __align__(16) uint32_t sched[160];  // the message in every round's order
-  uint32_t msg[16];
-  uint32_t sigma[5][32];  // sched entry lane + 32 j is word sigma[j][lane]
+  __align__(16) uint32_t sched[160];  // the message in kSigma's order
+  uint32_t msg[16], out[8];
+  uint32_t sigma[160];
 };
 
-// One compression by a warp (every lane alike) of the block in H.msg, as a loop over the rounds: the
-// unrolled form's 18 KB of instructions are fetched anew every time other code ran in between (2,630
-// cycles a compression in a round; the loop takes about 1,800). The lanes lay the message out in
-// every round's order first.
-__device__ __forceinline__ void warp_compress(Hash& H, uint32_t h[8], uint32_t t, bool last) {
-  const uint32_t lane = threadIdx.x & 31;
+// Compresses the block in H.msg into the chaining value in H.out, by one warp: every four lanes alike,
+// lane q the state's column q (h0 = v[q], h1 = v[4 + q]), the diagonals by rotating the rows among the
+// four. 56 instructions a half round, 40 of them on the ALU pipe, hold a lone lane's compression at
+// 1,672 cycles (2,430 as a loop that reads the message from shared memory, 2,630 unrolled where other
+// code ran in between and its 18 KB are fetched anew); a lane's 14 leave the latency of the step and
+// of three shuffles, and the loop's few instructions stay in the cache. init: start from the
+// parameter block.
+__device__ __forceinline__ void warp_compress(Hash& H, bool init, uint32_t t, bool last) {
+  const uint32_t lane = threadIdx.x & 31, q = lane & 3;
   __syncwarp();
 #pragma unroll
-  for (int j = 0; j < 5; j++) H.sched[lane + 32 * j] = H.msg[H.sigma[j][lane]];
+  for (int j = 0; j < 5; j++) H.sched[lane + 32 * j] = H.msg[H.sigma[lane + 32 * j]];
+  const uint32_t iv0 = q < 2 ? (q == 0 ? b2s_iv(0) : b2s_iv(1)) : (q == 2 ? b2s_iv(2) : b2s_iv(3));
+  const uint32_t iv1 = q < 2 ? (q == 0 ? b2s_iv(4) : b2s_iv(5)) : (q == 2 ? b2s_iv(6) : b2s_iv(7));
+  const uint32_t h0 = init ? iv0 ^ (q == 0 ? 0x01010020u : 0u) : H.out[q], h1 = init ? iv1 : H.out[4 + q];
+  uint32_t a = h0, b = h1, c = iv0, d = iv1 ^ (q == 0 ? t : q == 2 && last ? 0xffffffffu : 0u);
   __syncwarp();
-  uint32_t v0 = h[0], v1 = h[1], v2 = h[2], v3 = h[3], v4 = h[4], v5 = h[5], v6 = h[6], v7 = h[7];
-  uint32_t v8 = b2s_iv(0), v9 = b2s_iv(1), v10 = b2s_iv(2), v11 = b2s_iv(3);
-  uint32_t v12 = b2s_iv(4) ^ t, v13 = b2s_iv(5), v14 = last ? ~b2s_iv(6) : b2s_iv(6), v15 = b2s_iv(7);
-  const uint4* sched = reinterpret_cast<const uint4*>(H.sched);
-  uint4 a = sched[0], b = sched[1], c = sched[2], d = sched[3];
-#pragma unroll 1
-  for (int r = 0; r < 10; r++) {
-    const uint32_t m[16] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
-    const int n = r < 9 ? 4 * (r + 1) : 0;
-    a = sched[n], b = sched[n + 1], c = sched[n + 2], d = sched[n + 3];
-    CS_B2S_G_CHAIN(v0, v4, v8, v12, m[0], m[1])
-    CS_B2S_G_CHAIN(v1, v5, v9, v13, m[2], m[3])
-    CS_B2S_G_CHAIN(v2, v6, v10, v14, m[4], m[5])
-    CS_B2S_G_CHAIN(v3, v7, v11, v15, m[6], m[7])
-    CS_B2S_G_CHAIN(v0, v5, v10, v15, m[8], m[9])
-    CS_B2S_G_CHAIN(v1, v6, v11, v12, m[10], m[11])
-    CS_B2S_G_CHAIN(v2, v7, v8, v13, m[12], m[13])
-    CS_B2S_G_CHAIN(v3, v4, v9, v14, m[14], m[15])
+  const uint4* sched = reinterpret_cast<const uint4*>(H.sched) + q;
+  const int up = (int)((lane & 28) | ((q + 1) & 3)), across = (int)(lane ^ 2), down = (int)((lane & 28) | ((q + 3) & 3));
+  uint4 m = sched[0];
+#pragma unroll 2
+  for (int r = 1; r <= 10; r++) {
+    const uint4 n = sched[r < 10 ? 4 * r : 0];
+    CS_B2S_G_CHAIN(a, b, c, d, m.x, m.y)
+    b = __shfl_sync(0xffffffffu, b, up);
+    c = __shfl_sync(0xffffffffu, c, across);
+    d = __shfl_sync(0xffffffffu, d, down);
+    CS_B2S_G_CHAIN(a, b, c, d, m.z, m.w)
+    b = __shfl_sync(0xffffffffu, b, down);
+    c = __shfl_sync(0xffffffffu, c, across);
+    d = __shfl_sync(0xffffffffu, d, up);
+    m = n;
   }
-  h[0] ^= v0 ^ v8;
-  h[1] ^= v1 ^ v9;
-  h[2] ^= v2 ^ v10;
-  h[3] ^= v3 ^ v11;
-  h[4] ^= v4 ^ v12;
-  h[5] ^= v5 ^ v13;
-  h[6] ^= v6 ^ v14;
-  h[7] ^= v7 ^ v15;
+  if (lane < 4) {
+    H.out[q] = h0 ^ a ^ c;
+    H.out[4 + q] = h1 ^ b ^ d;
+  }
   __syncwarp();
 }
 
@@ -152,39 +161,35 @@ __device__ __forceinline__ void warp_compress(Hash& H, uint32_t h[8], uint32_t t
 __device__ __noinline__ void warp_mix(GkrState& S, Hash& H, const qm31* felts, uint32_t n) {
   const uint32_t lane = threadIdx.x & 31, words = 4 * n, len = 32 + 16 * n;
   const uint32_t* f = reinterpret_cast<const uint32_t*>(felts);
-  uint32_t h[8];
-  b2s_init(h);
   if (lane < 16) H.msg[lane] = lane < 8 ? S.chan[lane] : lane - 8 < words ? f[lane - 8] : 0;
   const bool two = len > 64;
 #pragma unroll 1
   for (int block = 0; block < (two ? 2 : 1); block++) {
     if (block == 1 && lane < 16) H.msg[lane] = lane < 8 && 8 + lane < words ? f[8 + lane] : 0;
     const bool last = block == (two ? 1 : 0);
-    warp_compress(H, h, last ? len : 64, last);
+    warp_compress(H, block == 0, last ? len : 64, last);
   }
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < 8; i++) S.chan[i] = h[i];
-    S.chan[8] = 0;
-  }
+  if (lane < 9) S.chan[lane] = lane < 8 ? H.out[lane] : 0;
   __syncwarp();
 }
 
 __device__ __noinline__ qm31 warp_draw(GkrState& S, Hash& H) {
   const uint32_t lane = threadIdx.x & 31;
   uint32_t h[8], state[9], felt[4];
-  b2s_init(h);
   if (lane < 16) H.msg[lane] = lane < 9 ? S.chan[lane] : 0;
-  warp_compress(H, h, kChannelDrawBytes, true);
+  warp_compress(H, true, kChannelDrawBytes, true);
+#pragma unroll
+  for (int i = 0; i < 8; i++) h[i] = H.out[i];
   state[8] = 0;
   channel_after_draw(state, h, felt);
+  __syncwarp();
   if (lane == 0) S.chan[8] += 1;
   __syncwarp();
   return q_make4(felt);
 }
 
 __device__ void hash_setup(Hash& H) {
-  for (uint32_t e = threadIdx.x; e < 160; e += blockDim.x) H.sigma[e >> 5][e & 31] = kSigma[e];
+  for (uint32_t e = threadIdx.x; e < 160; e += blockDim.x) H.sigma[e] = kSigma[e];
 }
 
 // One copy of the product's code for the latency-bound parts (their inlined products together would
@@ -227,7 +232,7 @@ __device__ __forceinline__ void make_poly(const GkrState& S, InstState& I, unsig
       b = s == 0 ? I.cu[t] : s == 1 ? I.lcu[t] : s == 2 ? I.cv[t] : I.lcv[t];
     } else if (s == 4) {
       a = I.claim;
-      b = S.w[layer - round][t];
+      b = S.row[layer - round].w[t];
     }
     p = mul(a, b);
     p = qm31_add(qm31_add(qm31_add(p, q_shfl(p, (lane + 4) & 31)), qm31_add(q_shfl(p, (lane + 8) & 31), q_shfl(p, (lane + 12) & 31))),
@@ -296,9 +301,9 @@ __device__ __forceinline__ void advance(const GkrState& S, InstState& I, uint32_
     a = I.poly[lane];
     b = lane == 1 ? x : lane == 2 ? x2 : x3;
   } else if (lane < 8) {
-    b = S.u[k][lane - 4];
+    b = S.row[k].u[lane - 4];
   } else if (lane < 12) {
-    b = S.v[k][lane - 8];
+    b = S.row[k].v[lane - 8];
   }
   const qm31 m3 = mul(a, b);
   const qm31 claim = qm31_add(qm31_add(I.poly[0], q_shfl(m3, 1)), qm31_add(q_shfl(m3, 2), q_shfl(m3, 3)));
@@ -319,91 +324,95 @@ __device__ __forceinline__ void advance_all(const GkrProgram& g, const GkrState&
     if (inst[i].delta <= layer) advance(S, inst[i], layer, round);
 }
 
-// The layer's first half: the claims of the instances that join (their output layer's values), every
-// claim into the channel, the round tables of the point y, the two draws and the sum-check claims.
-// One warp.
-__device__ void begin_layer(const GkrProgram& g, GkrState& S, InstState* inst, Hash& H, uint32_t layer) {
+// The round tables of the point y (lane j: the row of k = layer - j, from y[j]). One warp.
+__device__ void layer_tables(GkrState& S, uint32_t layer) {
   const uint32_t lane = threadIdx.x & 31;
-  for (uint32_t i = lane; i < g.n_inst; i += 32) {
-    InstState& I = inst[i];
-    if (I.delta != layer) continue;
-    const uint32_t* const* c = g.out0 + 8 * i;
-    uint32_t n = 0;
-    if (c[0] != nullptr) I.out[n++] = qm31_make(*c[0], *c[1], *c[2], *c[3]);
-    I.out[n++] = qm31_make(*c[4], *c[5], *c[6], *c[7]);
-    I.n_out = n;
-    for (uint32_t t = 0; t < n; t++) q_put(g.outputs + 8 * i + 4 * t, I.out[t]);
-  }
-  __syncwarp();
-  for (uint32_t i = 0; i < g.n_inst; i++)
-    if (inst[i].delta <= layer) warp_mix(S, H, inst[i].out, inst[i].n_out);
-  // lane j: the tables of k = layer - j, from y[j]
-  {
-    const bool on = lane < layer;
-    const qm31 y = on ? S.y[lane] : q_zero();
-    const qm31 one_y = qm31_sub(q_one(), y);
-    qm31 prefix = one_y;  // prod_{t <= j} (1 - y_t)
+  const bool on = lane < layer;
+  const qm31 y = on ? S.y[lane] : q_zero();
+  const qm31 one_y = qm31_sub(q_one(), y);
+  qm31 prefix = one_y;  // prod_{t <= j} (1 - y_t)
 #pragma unroll 1
-    for (int off = 1; off < 32; off <<= 1) {
-      const qm31 m = mul(prefix, q_shfl(prefix, (lane - off) & 31));
-      if (lane >= (uint32_t)off) prefix = m;
-    }
-    const qm31 d = qm31_sub(one_y, y);
-    const qm31 pd = mul(prefix, d);
-    const qm31 inv = qm31_inv(pd);
-    const qm31 a = mul(inv, d);                       // 1 / prefix
-    const qm31 b = mul(one_y, mul(inv, prefix));      // (1 - y) / (1 - 2 y)
-    const qm31 x0 = qm31_neg(b), x1 = qm31_sub(q_one(), b), x2 = qm31_add_m31(x1, 1);
-    const qm31 x01 = mul(x0, x1), x012 = mul(x01, x2);
-    const qm31 inv3 = qm31_inv(x012);
-    const qm31 inv01 = mul(inv3, x2);
-    const qm31 i0 = mul(inv01, x1), i1 = mul(inv01, x0), i2 = mul(inv3, x01);  // 1 / (x - b)
-    const qm31 e0 = mul(a, one_y);                                                         // a eq(0, y)
-    const qm31 e2 = mul(a, qm31_add_m31(qm31_add(q_double(y), y), P - 1));                 // a eq(2, y)
-    // q0 = f0 al, q1 = claim i1 - f0 be, q2 = f2 ga; c2 = (q2 - 2 q1 + q0) / 2, c1 = q1 - q0 - c2;
-    // the polynomial is (t - b) (q0 + c1 t + c2 t^2)
-    const qm31 al = mul(e0, i0), be = mul(e0, i1), ga = mul(e2, i2);
-    const uint32_t half = (P + 1) / 2;
-    const qm31 al2 = qm31_mul_m31(al, half), ga2 = qm31_mul_m31(ga, half), be2 = q_double(be), i1x2 = q_double(i1);
-    if (on) {
-      const uint32_t k = layer - lane;
-      auto put = [&](qm31* o, qm31 q0, qm31 c1, qm31 c2) {
-        o[0] = qm31_neg(mul(b, q0));
-        o[1] = qm31_sub(q0, mul(b, c1));
-        o[2] = qm31_sub(c1, mul(b, c2));
-        o[3] = c2;
-      };
-      put(S.u[k], al, qm31_neg(qm31_add(be2, qm31_add(al, al2))), qm31_add(al2, be));
-      put(S.v[k], q_zero(), qm31_neg(ga2), ga2);
-      put(S.w[k], q_zero(), i1x2, qm31_neg(i1));
-      if (q_is_zero(pd) || q_is_zero(x012)) S.err = 1;
-    }
+  for (int off = 1; off < 32; off <<= 1) {
+    const qm31 m = mul(prefix, q_shfl(prefix, (lane - off) & 31));
+    if (lane >= (uint32_t)off) prefix = m;
   }
-  __syncwarp();
-  const qm31 alpha = warp_draw(S, H);
-  const qm31 lam = warp_draw(S, H);
-  if (lane == 0) {
-    S.alpha = alpha;
-    S.lam = lam;
-  }
-  qm31 apow = q_one();
-  for (uint32_t i = 0; i < g.n_inst; i++) {
-    InstState& I = inst[i];
-    if (I.delta > layer) continue;
-    qm31 c = I.out[I.n_out - 1];
-    if (I.n_out == 2) c = qm31_add(mul(c, lam), I.out[0]);
-    // an instance that joined delta layers late counts every point 2^delta times
-    c = qm31_mul_m31(c, 1u << I.delta);
+  const qm31 d = qm31_sub(one_y, y);
+  const qm31 pd = mul(prefix, d);
+  const qm31 inv = qm31_inv(pd);
+  const qm31 a = mul(inv, d);                   // 1 / prefix
+  const qm31 b = mul(one_y, mul(inv, prefix));  // (1 - y) / (1 - 2 y)
+  const qm31 x0 = qm31_neg(b), x1 = qm31_sub(q_one(), b), x2 = qm31_add_m31(x1, 1);
+  const qm31 x01 = mul(x0, x1), x012 = mul(x01, x2);
+  const qm31 inv3 = qm31_inv(x012);
+  const qm31 inv01 = mul(inv3, x2);
+  const qm31 i0 = mul(inv01, x1), i1 = mul(inv01, x0), i2 = mul(inv3, x01);  // 1 / (x - b)
+  const qm31 e0 = mul(a, one_y);                                             // a eq(0, y)
+  const qm31 e2 = mul(a, qm31_add_m31(qm31_add(q_double(y), y), P - 1));     // a eq(2, y)
+  // q0 = f0 al, q1 = claim i1 - f0 be, q2 = f2 ga; c2 = (q2 - 2 q1 + q0) / 2, c1 = q1 - q0 - c2;
+  // the polynomial is (t - b) (q0 + c1 t + c2 t^2)
+  const qm31 al = mul(e0, i0), be = mul(e0, i1), ga = mul(e2, i2);
+  const uint32_t half = (P + 1) / 2;
+  const qm31 al2 = qm31_mul_m31(al, half), ga2 = qm31_mul_m31(ga, half), be2 = q_double(be), i1x2 = q_double(i1);
+  auto put = [&](qm31* o, qm31 q0, qm31 c1, qm31 c2) {
+    const qm31 o0 = qm31_neg(mul(b, q0)), o1 = qm31_sub(q0, mul(b, c1)), o2 = qm31_sub(c1, mul(b, c2));
+    if (on) o[0] = o0, o[1] = o1, o[2] = o2, o[3] = c2;
+  };
+  auto& row = S.row[on ? layer - lane : 0];
+  put(row.u, al, qm31_neg(qm31_add(be2, qm31_add(al, al2))), qm31_add(al2, be));
+  put(row.v, q_zero(), qm31_neg(ga2), ga2);
+  put(row.w, q_zero(), i1x2, qm31_neg(i1));
+  if (on && (q_is_zero(pd) || q_is_zero(x012))) S.err = 1;
+}
+
+// The layer's first half: the claims of the instances that join (their output layer's values), every
+// claim into the channel and the two draws by one warp, the round tables by another, then the
+// sum-check claims. The block (two warps at least); ends with a barrier.
+__device__ void begin_layer(const GkrProgram& g, GkrState& S, InstState* inst, Hash& H, uint32_t layer) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp == 1) layer_tables(S, layer);
+  if (warp == 0) {
+    for (uint32_t i = lane; i < g.n_inst; i += 32) {
+      InstState& I = inst[i];
+      if (I.delta != layer) continue;
+      const uint32_t* const* c = g.out0 + 8 * i;
+      uint32_t n = 0;
+      if (c[0] != nullptr) I.out[n++] = qm31_make(*c[0], *c[1], *c[2], *c[3]);
+      I.out[n++] = qm31_make(*c[4], *c[5], *c[6], *c[7]);
+      I.n_out = n;
+      for (uint32_t t = 0; t < n; t++) q_put(g.outputs + 8 * i + 4 * t, I.out[t]);
+    }
+    __syncwarp();
+    for (uint32_t i = 0; i < g.n_inst; i++)
+      if (inst[i].delta <= layer) warp_mix(S, H, inst[i].out, inst[i].n_out);
+    const qm31 alpha = warp_draw(S, H);
+    const qm31 lam = warp_draw(S, H);
     if (lane == 0) {
-      I.claim = c;
-      I.corr = q_one();
-      I.apow = apow;
+      S.alpha = alpha;
+      S.lam = lam;
     }
-    apow = mul(apow, alpha);
-    put_tables(I, lane >= 4 && lane < 8 ? S.u[layer][lane - 4] : lane >= 8 && lane < 12 ? S.v[layer][lane - 8] : q_zero(),
-               lam);
+    qm31 apow = q_one();
+    for (uint32_t i = 0; i < g.n_inst; i++) {
+      InstState& I = inst[i];
+      if (I.delta > layer) continue;
+      qm31 c = I.out[I.n_out - 1];
+      if (I.n_out == 2) c = qm31_add(mul(c, lam), I.out[0]);
+      // an instance that joined delta layers late counts every point 2^delta times
+      c = qm31_mul_m31(c, 1u << I.delta);
+      if (lane == 0) {
+        I.claim = c;
+        I.corr = q_one();
+        I.apow = apow;
+      }
+      if (i + 1 < g.n_inst) apow = mul(apow, alpha);
+    }
   }
-  __syncwarp();
+  __syncthreads();
+  for (uint32_t i = warp; i < g.n_inst; i += blockDim.x >> 5)
+    if (inst[i].delta <= layer)
+      put_tables(inst[i],
+                 lane >= 4 && lane < 8 ? S.row[layer].u[lane - 4] : lane >= 8 && lane < 12 ? S.row[layer].v[lane - 8] : q_zero(),
+                 S.lam);
+  __syncthreads();
 }
 
 // ------------------------------------------------------------ the sums of a round
@@ -556,6 +565,48 @@ __device__ void store_block(const GkrProgram& g, const Block& B) {
   if (B.inst != g.inst) copy_words(g.inst, B.inst, sizeof(InstState) * g.n_inst);
 }
 
+// Programmatic dependent launch: a kernel of the chain may start while the one before it drains, and
+// waits here for its end before it reads what that one wrote. Released to the next kernel right after.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+__device__ __forceinline__ void copy_async(void* dst, const void* src, size_t bytes) {  // multiples of 16 bytes
+  for (uint32_t k = threadIdx.x; k < bytes / 16; k += blockDim.x)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(
+                     static_cast<unsigned char*>(dst) + 16 * k)),
+                 "l"(static_cast<const unsigned char*>(src) + 16 * k));
+}
+// The part of the state that ending a round reads, fetched while the block sums its terms.
+__device__ Block prefetch_block(const GkrProgram& g, unsigned char* smem, uint32_t layer, uint32_t round) {
+  Block B;
+  B.S = reinterpret_cast<GkrState*>(smem);
+  B.H = reinterpret_cast<Hash*>(smem + sizeof(GkrState));
+  B.inst = g.inst;
+  B.acc = g.acc;
+  const uint32_t k = layer - round;
+  copy_async(B.S, g.state, offsetof(GkrState, y));
+  copy_async(&B.S->y[round], &g.state->y[round], sizeof(qm31));
+  copy_async(&B.S->row[k - 1], &g.state->row[k - 1], 2 * sizeof(B.S->row[0]));
+  if (g.n_inst <= kSharedInst) {
+    unsigned char* p = smem + sizeof(GkrState) + sizeof(Hash);
+    B.acc = reinterpret_cast<unsigned long long*>(p);
+    B.inst = reinterpret_cast<InstState*>(p + 16 * sizeof(unsigned long long) * g.n_inst);
+    copy_async(B.inst, g.inst, sizeof(InstState) * g.n_inst);
+    for (uint32_t j = threadIdx.x; j < 16 * g.n_inst; j += blockDim.x) B.acc[j] = 0;
+  }
+  B.rest = nullptr;
+  return B;
+}
+// What ending a round changed.
+__device__ void store_round(const GkrProgram& g, const Block& B, uint32_t round) {
+  __syncthreads();
+  copy_words(g.state, B.S, offsetof(GkrState, y));
+  copy_words(&g.state->sc[round], &B.S->sc[round], sizeof(qm31));
+  if (B.inst != g.inst) copy_words(g.inst, B.inst, sizeof(InstState) * g.n_inst);
+}
+
 __device__ __forceinline__ void add_to(unsigned long long* acc, qm31 v) {
   atomicAdd(acc + 0, (unsigned long long)v.a.a);
   atomicAdd(acc + 1, (unsigned long long)v.a.b);
@@ -575,6 +626,9 @@ __global__ void __launch_bounds__(kRoundThreads) gkr_round_kernel(const GkrProgr
   __shared__ bool last;
   __shared__ qm31 part[4][kRoundThreads / 32];
   const uint32_t i = blockIdx.y, delta = g.inst[i].delta, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  hash_setup(*reinterpret_cast<Hash*>(smem + sizeof(GkrState)));
+  chain_wait();
+  const Block B = prefetch_block(g, smem, layer, round);
   if (delta <= round) {
     const Sums s = round_terms(g.cols[(size_t)layer * g.n_inst + i], round - delta, 1u << (layer - round - 1),
                                blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, g.eq, 1u << (layer - 1),
@@ -590,12 +644,12 @@ __global__ void __launch_bounds__(kRoundThreads) gkr_round_kernel(const GkrProgr
       __threadfence();
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(g.counter, 1u) == gridDim.x * gridDim.y - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  const Block B = load_block(g, smem);
   for (uint32_t j = 0; j < g.n_inst; j++) {
     if (B.inst[j].delta > round) continue;
     // thread 4 b + k adds sum k of the blocks b, b + 32, ...
@@ -611,7 +665,7 @@ __global__ void __launch_bounds__(kRoundThreads) gkr_round_kernel(const GkrProgr
   __syncthreads();
   finish_round(g, *B.S, B.inst, B.acc, *B.H, layer, round);
   advance_all(g, *B.S, B.inst, layer, round);
-  store_block(g, B);
+  store_round(g, B, round);
   if (threadIdx.x == 0) *g.counter = 0;
 }
 
@@ -717,28 +771,32 @@ __device__ void tail_round(const GkrProgram& g, const Block& B, uint32_t* shared
 __device__ void end_layer(const GkrProgram& g, const Block& B, uint32_t* shared, uint32_t layer) {
   const uint32_t lane = threadIdx.x & 31;
   GkrState& S = *B.S;
-  for (uint32_t i = lane; i < g.n_inst; i += 32) {
+  // a lane per (instance, column, value); a mask without numerators has the denominators first
+  for (uint32_t idx = lane; idx < 4 * g.n_inst; idx += 32) {
+    const uint32_t i = idx >> 2, c = (idx >> 1) & 1, j = idx & 1;
     InstState& I = B.inst[i];
     if (I.delta > layer) continue;
     const TailCols C = tail_cols(g, shared, layer, i, layer - I.delta, false);
-    uint32_t n = 0;
-    if (C.L->kind == CS_GKR_LOGUP_SINGLES) I.poly[0] = I.poly[1] = q_one(), n = 2;
-    for (int c = 0; c < 2; c++) {
-      if (!C.has(c)) continue;
-      for (uint32_t j = 0; j < 2; j++) {
-        qm31 v[2];
-        for (int h = 0; h < 2; h++) {
-          uint32_t w[4] = {0, 0, 0, 0};
-          for (int k = 0; k < (C.base(c) && C.fixes == 1 ? 1 : 4); k++)
-            if (h == 0 || C.fixes > 0) w[k] = C.before(c, k)[j + 2 * h];
-          v[h] = q_make4(w);
-        }
-        I.poly[n++] = C.fixes > 0 ? q_lerp(v[0], v[1], S.x) : v[0];
+    const bool ones = C.L->kind == CS_GKR_LOGUP_SINGLES;
+    if (j == 0 && c == 1) I.n_out = C.has(0) || ones ? 2 : 1;
+    qm31 m = q_one();
+    if (C.has(c)) {
+      qm31 v[2];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if ((k == 0 || !(C.base(c) && C.fixes == 1)) && (h == 0 || C.fixes > 0)) w[k] = C.before(c, k)[j + 2 * h];
+        v[h] = q_make4(w);
       }
+      m = C.fixes > 0 ? q_lerp(v[0], v[1], S.x) : v[0];
+    } else if (!ones) {
+      continue;
     }
-    uint32_t* o = g.masks + 16 * ((size_t)layer * g.n_inst + i);
-    for (uint32_t t = 0; t < n; t++) q_put(o + 4 * t, I.poly[t]);
-    I.n_out = n / 2;
+    const uint32_t t = C.has(0) || ones ? idx & 3 : j;
+    I.poly[t] = m;
+    q_put(g.masks + 16 * ((size_t)layer * g.n_inst + i) + 4 * t, m);
   }
   __syncwarp();
   for (uint32_t i = 0; i < g.n_inst; i++)
@@ -760,18 +818,17 @@ size_t tail_smem(uint32_t n_inst) {
   return block_bytes(n_inst) + (n_inst <= kSharedCols ? (size_t)n_inst * 32 * kTailTerms * sizeof(uint32_t) : 0);
 }
 
-// Rounds [round, layer) of `layer`, its masks, the next layer's claims and tables, and the whole of
-// the layers that follow while they have at most kTailRounds rounds; ends with the claims of the first
-// longer layer in place. begin: start with the first layer's claims.
+// Rounds [round, layer) of `layer` and its masks, and the whole of the layers that follow while they
+// have at most kTailRounds rounds. begin: start with the layer's claims.
 __global__ void __launch_bounds__(kTailThreads) gkr_tail_kernel(const GkrProgram g, uint32_t layer, uint32_t round,
                                                                 uint32_t begin) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint32_t eq[4][kTailTerms];
+  chain_wait();
   const Block B = load_block(g, smem);
   uint32_t* shared = g.n_inst <= kSharedCols ? reinterpret_cast<uint32_t*>(B.rest) : nullptr;
   if (begin) {
-    if (threadIdx.x < 32) begin_layer(g, *B.S, B.inst, *B.H, layer);
-    __syncthreads();
+    begin_layer(g, *B.S, B.inst, *B.H, layer);
   }
   for (;;) {
     const uint32_t entry = round;
@@ -804,17 +861,28 @@ __global__ void __launch_bounds__(kTailThreads) gkr_tail_kernel(const GkrProgram
     if (threadIdx.x < 32) end_layer(g, B, shared, layer);
     layer++;
     round = 0;
-    if (layer == g.n_layers) break;
-    if (threadIdx.x < 32) begin_layer(g, *B.S, B.inst, *B.H, layer);
+    if (layer == g.n_layers || layer > kTailRounds) break;
     __syncthreads();
-    if (layer > kTailRounds) break;
+    begin_layer(g, *B.S, B.inst, *B.H, layer);
   }
   store_block(g, B);
 }
 
-// The layer's eq column from the point in the state (eq_evals_kernel).
-__global__ void __launch_bounds__(256) gkr_layer_eq_kernel(const GkrState* state, uint32_t layer, const QOut out) {
-  eq_evals_block(qm31_sub(q_one(), state->y[0]), state->y + 1, layer - 1, out);
+// A long layer's start: block 0 makes the claims and tables, the others the layer's eq column from the
+// point in the state (eq_evals_kernel), 2^kEqChunkBits values each.
+__global__ void __launch_bounds__(256) gkr_start_kernel(const GkrProgram g, uint32_t layer, const QOut eq) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  chain_wait();
+  if (blockIdx.x == 0) {
+    const Block B = load_block(g, smem);
+    begin_layer(g, *B.S, B.inst, *B.H, layer);
+    // the point stays as it is: the other blocks read it
+    copy_words(g.state, B.S, offsetof(GkrState, y));
+    copy_words(g.state->row, B.S->row, sizeof(B.S->row));
+    if (B.inst != g.inst) copy_words(g.inst, B.inst, sizeof(InstState) * g.n_inst);
+    return;
+  }
+  eq_evals_block(blockIdx.x - 1, qm31_sub(q_one(), g.state->y[0]), g.state->y + 1, layer - 1, eq);
 }
 
 // ------------------------------------------------------------ host
@@ -823,7 +891,7 @@ __global__ void __launch_bounds__(256) gkr_layer_eq_kernel(const GkrState* state
 template <typename Kernel>
 cs_status allow_smem(Kernel kernel, size_t bytes, int which) {
   static std::mutex mu;
-  static bool done[2][kMaxDevices] = {};
+  static bool done[3][kMaxDevices] = {};
   int dev = 0;
   CS_CUDA(cudaGetDevice(&dev));
   CS_CHECK_ARG(dev >= 0 && dev < kMaxDevices, "gkr_prove_batch: device ordinal %d out of range", dev);
@@ -991,21 +1059,40 @@ cs_status gkr_prove_on_device(const std::vector<GkrInput>& inputs, uint32_t chan
   cs_status attr = allow_smem(gkr_tail_kernel, tail_smem(kSharedCols), 0);
   if (attr == CS_OK) attr = allow_smem(gkr_round_kernel, block_bytes(kSharedInst), 1);
   if (attr != CS_OK) return attr;
+  attr = allow_smem(gkr_start_kernel, block_bytes(kSharedInst), 2);
+  if (attr != CS_OK) return attr;
   gkr_tail_kernel<<<1, kTailThreads, tail_bytes, st>>>(g, 0, 0, 1);
   CS_LAUNCHED("gkr_tail_kernel");
+  // the rest is one chain of dependent launches
+  cudaLaunchAttribute dependent;
+  dependent.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  dependent.val.programmaticStreamSerializationAllowed = 1;
+  auto config = [&](dim3 grid, uint32_t threads, size_t smem) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &dependent;
+    c.numAttrs = 1;
+    return c;
+  };
   for (uint32_t l = kTailRounds + 1; l < n_layers; l++) {
     QOut e;
     for (int k = 0; k < 4; k++) e.c[k] = eq + ((size_t)k << (l - 1));
-    gkr_layer_eq_kernel<<<1u << (l - 1 - std::min(l - 1, kEqChunkBits)), 256, 0, st>>>(g.state, l, e);
-    CS_LAUNCHED("gkr_layer_eq_kernel");
+    cudaLaunchConfig_t c = config(dim3(1 + (1u << (l - 1 - std::min(l - 1, kEqChunkBits)))), 256, round_bytes);
+    CS_CUDA(cudaLaunchKernelEx(&c, gkr_start_kernel, (const GkrProgram)g, l, (const QOut)e));
+    note_launch();
     for (uint32_t r = 0; r + kTailRounds < l; r++) {
       const uint64_t terms = 1ull << (l - r - 1);
       const uint32_t blocks = (uint32_t)std::min<uint64_t>((terms + kRoundThreads - 1) / kRoundThreads, 152 * 8);
-      gkr_round_kernel<<<dim3(blocks, n_inst), kRoundThreads, round_bytes, st>>>(g, l, r);
-      CS_LAUNCHED("gkr_round_kernel");
+      c = config(dim3(blocks, n_inst), kRoundThreads, round_bytes);
+      CS_CUDA(cudaLaunchKernelEx(&c, gkr_round_kernel, (const GkrProgram)g, l, r));
+      note_launch();
     }
-    gkr_tail_kernel<<<1, kTailThreads, tail_bytes, st>>>(g, l, l - kTailRounds, 0);
-    CS_LAUNCHED("gkr_tail_kernel");
+    c = config(dim3(1), kTailThreads, tail_bytes);
+    CS_CUDA(cudaLaunchKernelEx(&c, gkr_tail_kernel, (const GkrProgram)g, l, l - kTailRounds, 0u));
+    note_launch();
   }
   std::vector<unsigned char> back(at_partial);
   CS_CUDA(cudaMemcpyAsync(back.data(), dev, back.size(), cudaMemcpyDeviceToHost, st));
