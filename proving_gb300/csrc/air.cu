@@ -31,37 +31,77 @@ __device__ __forceinline__ uint32_t fold64(uint64_t v) {
   return m31_reduce_once((uint32_t)((t & P) + (t >> 31)));
 }
 
-__global__ void __launch_bounds__(256) wide_fib_composition_kernel(const __grid_constant__ WideFibParams p,
-                                                                    uint32_t* a0, uint32_t* a1, uint32_t* a2,
-                                                                    uint32_t* a3) {
-  const uint32_t n = 1u << p.eval_log;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+// A warp takes 32 rows and one of `split` runs of the constraints; the runs of a row group are warps of
+// one block and meet in shared memory. Columns are loaded eight ahead of the constraint that reads
+// them: one at a time, the loop waited for every load (36 us for the 98 constraints of 2^15 rows).
+constexpr int kFibWarps = 8, kFibAhead = 8;
+
+__global__ void __launch_bounds__(32 * kFibWarps) wide_fib_composition_kernel(const __grid_constant__ WideFibParams p,
+                                                                              uint32_t split, uint32_t* a0,
+                                                                              uint32_t* a1, uint32_t* a2,
+                                                                              uint32_t* a3) {
+  __shared__ uint32_t part[kFibWarps][4][32];
+  const uint32_t n = 1u << p.eval_log, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t run = warp & (split - 1), group = warp / split, groups = kFibWarps / split;
+  const uint32_t n_con = p.n_cols - 2, per = (n_con + split - 1) / split;
+  const uint32_t k0 = min(n_con, run * per), k1 = min(n_con, k0 + per);
+  uint32_t* const out[4] = {a0, a1, a2, a3};
+  for (uint32_t base = blockIdx.x * groups * 32; base < n; base += gridDim.x * groups * 32) {
+    const uint32_t r = base + group * 32 + lane;
     // Lazy sums: each weight x constraint product is below 2^62 and is added unreduced (one
     // 64-bit multiply-add per coordinate); folding every four constraints keeps the sums below
     // 2^64 (a fold leaves less than 2^34). Each column is squared once, for the constraint that
     // reads it as b and the next one that reads it as a.
     uint64_t acc[4] = {0, 0, 0, 0};
-    uint32_t sa = m31_sqr(__ldg(p.cols[0] + r)), sb = m31_sqr(__ldg(p.cols[1] + r));
-    for (uint32_t k = 0; k + 2 < p.n_cols; k++) {
-      const uint32_t c = __ldg(p.cols[k + 2] + r);
-      const uint32_t cons = m31_sub(c, m31_add(sa, sb));
-      const qm31 w = p.rc[k];
-      acc[0] += (uint64_t)w.a.a * cons;
-      acc[1] += (uint64_t)w.a.b * cons;
-      acc[2] += (uint64_t)w.b.a * cons;
-      acc[3] += (uint64_t)w.b.b * cons;
-      if ((k & 3) == 3) {
+    if (r < n && k0 < k1) {
+      uint32_t sa = m31_sqr(__ldg(p.cols[k0] + r)), sb = m31_sqr(__ldg(p.cols[k0 + 1] + r));
+      uint32_t next[kFibAhead];
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[j] = (acc[j] & P) + (acc[j] >> 31);
+      for (int j = 0; j < kFibAhead; j++) next[j] = k0 + j < k1 ? __ldg(p.cols[k0 + j + 2] + r) : 0;
+      for (uint32_t k = k0; k < k1; k += kFibAhead) {
+        uint32_t cur[kFibAhead];
+#pragma unroll
+        for (int j = 0; j < kFibAhead; j++) {
+          cur[j] = next[j];
+          next[j] = k + kFibAhead + j < k1 ? __ldg(p.cols[k + kFibAhead + j + 2] + r) : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < kFibAhead; j++) {
+          if (k + j < k1) {
+            const uint32_t cons = m31_sub(cur[j], m31_add(sa, sb));
+            const qm31 w = p.rc[k + j];
+            acc[0] += (uint64_t)w.a.a * cons;
+            acc[1] += (uint64_t)w.a.b * cons;
+            acc[2] += (uint64_t)w.b.a * cons;
+            acc[3] += (uint64_t)w.b.b * cons;
+          }
+          if ((j & 3) == 3) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) acc[c] = (acc[c] & P) + (acc[c] >> 31);
+          }
+          sa = sb;
+          sb = m31_sqr(cur[j]);
+        }
       }
-      sa = sb;
-      sb = m31_sqr(c);
     }
-    const uint32_t d = p.den[r >> p.trace_log];
-    a0[r] = m31_add(a0[r], m31_mul(fold64(acc[0]), d));
-    a1[r] = m31_add(a1[r], m31_mul(fold64(acc[1]), d));
-    a2[r] = m31_add(a2[r], m31_mul(fold64(acc[2]), d));
-    a3[r] = m31_add(a3[r], m31_mul(fold64(acc[3]), d));
+    uint32_t v[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) v[c] = fold64(acc[c]);
+    if (split > 1) {
+#pragma unroll
+      for (int c = 0; c < 4; c++) part[warp][c][lane] = v[c];
+      __syncthreads();
+      if (run == 0)
+        for (uint32_t w = 1; w < split; w++)
+#pragma unroll
+          for (int c = 0; c < 4; c++) v[c] = m31_add(v[c], part[warp + w][c][lane]);
+    }
+    if (run == 0 && r < n) {
+      const uint32_t d = p.den[r >> p.trace_log];
+#pragma unroll
+      for (int c = 0; c < 4; c++) out[c][r] = m31_add(out[c][r], m31_mul(v[c], d));
+    }
+    if (split > 1) __syncthreads();
   }
 }
 
@@ -135,9 +175,13 @@ extern "C" cs_status cs_wide_fib_composition(const uint32_t* const* h_cols, uint
   }
   for (int c = 0; c < 4; c++) CS_CHECK_ARG(h_accum[c] != nullptr, "wide_fib_composition: null accumulator");
   const uint32_t n = 1u << eval_log;
-  const uint32_t blocks = std::max(1u, std::min((n + 255) / 256, 152u * 8));
-  wide_fib_composition_kernel<<<blocks, 256, 0, to_stream(stream)>>>(p, h_accum[0], h_accum[1], h_accum[2],
-                                                                     h_accum[3]);
+  // runs of eight constraints and more, as many as it takes for the chip's 2048 threads an SM
+  uint32_t split = 1;
+  while (split < (uint32_t)kFibWarps && (uint64_t)n * split < 152ull * 2048 && (n_cols - 2) / (2 * split) >= 8) split *= 2;
+  const uint32_t rows = 32 * (kFibWarps / split);
+  const uint32_t blocks = std::max(1u, std::min((n + rows - 1) / rows, 152u * 8));
+  wide_fib_composition_kernel<<<blocks, 32 * kFibWarps, 0, to_stream(stream)>>>(p, split, h_accum[0], h_accum[1],
+                                                                               h_accum[2], h_accum[3]);
   CS_LAUNCHED("wide_fib_composition_kernel");
   return CS_OK;
 }

@@ -485,13 +485,12 @@ __device__ __forceinline__ void circle_stage(const FftPass& p, uint32_t g, uint3
   }
 }
 
-// x 2^k mod P for a canonic x: a rotation of its 31 bits.
-__device__ __forceinline__ uint32_t mul_pow2(uint32_t x, uint32_t k) { return __funnelshift_l(x << 1, x, k) & P; }
-
-// Register budget: 64 registers for 32 values a thread (1024 threads an SM), 40 for 16 or fewer.
+// Register budget: 64 registers for 32 values a thread (1024 threads an SM), 40 for 16 or fewer; for 64
+// values 96 in the contiguous pass's 128-thread blocks and 128 in the strided one's (80 there spill:
+// 32 x 2^22 as (11, 11) 688 against 640 us).
 template <int TB>
 constexpr int direct_min_blocks(int threads) {
-  const int b = (TB >= 6 ? 512 : TB == 5 ? 1024 : 1536) / threads;
+  const int b = (TB >= 6 ? (threads == 256 ? 512 : 640) : TB == 5 ? 1024 : 1536) / threads;
   return b < 24 ? b : 24;
 }
 
@@ -587,7 +586,7 @@ __global__ void __launch_bounds__(32 * kContigWarps, direct_min_blocks<T - T / 2
     if (p.scale) {
       const uint32_t k = __ffs(p.scale) - 1;
 #pragma unroll
-      for (int j = 0; j < V; j++) v[j] = mul_pow2(v[j], k);
+      for (int j = 0; j < V; j++) v[j] = m31_mul_pow2(v[j], k);
     }
 #pragma unroll
     for (int j = 0; j < V; j++) q[j << TA] = v[j];
@@ -620,7 +619,7 @@ constexpr uint32_t strided_tile_words() {
 template <int T, int EB>
 constexpr uint32_t strided_smem_words() {
   constexpr int TA = T / 2, TB = T - TA;
-  return strided_tile_words<T, EB>() + (((1u << EB) << TA) / 32) * ((1u << TB) + ((32u >> EB) << TB));
+  return strided_tile_words<T, EB>() + (1u << TB) + (((1u << EB) << TA) / 32) * ((32u >> EB) << TB);
 }
 
 // Layers [lo, lo + T), lo >= 3: a block owns the 2^T values of 8 neighbouring groups (32-byte runs
@@ -633,8 +632,9 @@ __global__ void __launch_bounds__((1 << EB) << (T / 2), direct_min_blocks<T - T 
   const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31;
   constexpr int RW = 32 >> EB;  // rows a warp
   const uint32_t e = t & ((1u << EB) - 1), ml = t >> EB;
-  uint32_t* tabB = smem + strided_tile_words<T, EB>() + warp * ((1u + RW) << TB);
-  uint32_t* tabA = tabB + (1 << TB);
+  // every warp writes the same words to the high stage's table, which depends on the block alone
+  uint32_t* tabB = smem + strided_tile_words<T, EB>();
+  uint32_t* tabA = tabB + (1 << TB) + warp * (RW << TB);
   // replicated reads (evaluate's first pass): the replicas of a tile are neighbouring blocks and
   // share its reads; otherwise neighbouring runs of the same lines are
   const uint32_t outer_bits = p.log_n - p.hi, run_bits = p.lo - EB;
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__((1 << EB) << (T / 2), direct_min_blocks<T - T 
     if (p.scale) {
       const uint32_t k = __ffs(p.scale) - 1;
 #pragma unroll
-      for (int j = 0; j < V; j++) v[j] = mul_pow2(v[j], k);
+      for (int j = 0; j < V; j++) v[j] = m31_mul_pow2(v[j], k);
     }
     uint32_t* q = dst + ((size_t)ml << p.lo);
 #pragma unroll

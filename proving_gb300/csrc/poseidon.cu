@@ -68,7 +68,7 @@ __device__ __forceinline__ void internal_matrix(uint32_t* s) {
 #pragma unroll
   for (int i = 1; i < kState; i++) sum = m31_add(sum, s[i]);
 #pragma unroll
-  for (int i = 0; i < kState; i++) s[i] = m31_add(m31_mul(s[i], 1u << (i + 1)), sum);
+  for (int i = 0; i < kState; i++) s[i] = m31_add(m31_mul_pow2(s[i], i + 1), sum);
 }
 
 __device__ __forceinline__ uint32_t pow5(uint32_t x) {
