@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import ctypes
 import threading
+from array import array
 from dataclasses import dataclass
 
 import numpy as np
@@ -24,7 +25,14 @@ P = (1 << 31) - 1
 M31_CIRCLE_LOG_ORDER = 31
 
 
+_data_ptr = torch.Tensor.data_ptr
+
+
 def _stream():
+    """torch's current stream. Asked of the runtime binding directly once CUDA is up:
+    torch.cuda.current_stream() builds a Stream object, 6 us of a call that launches one kernel."""
+    if torch.cuda.is_initialized():
+        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
@@ -36,14 +44,13 @@ def _ptr(t: torch.Tensor) -> int:
 def _ptr_table(ts) -> ctypes.Array:
     """Device pointers of the tensors (BaseColumn data: 1-D contiguous CUDA int32, checked when the
     column was made)."""
-    return (ctypes.c_void_p * max(1, len(ts)))(*[t.data_ptr() for t in ts])
+    ptrs = array("Q", map(_data_ptr, ts))
+    return (ctypes.c_void_p * len(ptrs)).from_buffer(ptrs) if ptrs else (ctypes.c_void_p * 1)()
 
 
 def _u32_table(vals) -> ctypes.Array:
-    arr = (ctypes.c_uint32 * max(1, len(vals)))()
-    for i, v in enumerate(vals):
-        arr[i] = int(v)
-    return arr
+    words = vals.tolist() if isinstance(vals, np.ndarray) else list(map(int, vals))
+    return (ctypes.c_uint32 * max(1, len(words)))(*words)
 
 
 def subgroup_gen(log_size: int) -> int:
@@ -317,7 +324,7 @@ class CudaBackend:
         n = 1 if not columns else 1 << lifting_log_size
         out = torch.empty((n, 8), dtype=torch.int32, device="cuda")
         tab = _ptr_table([c.data for c in columns])
-        logs = _u32_table([c.log_size for c in columns])
+        logs = _u32_table([c._log_size for c in columns])
         _lib.call("cs_merkle_build_leaves", tab, logs, len(columns), lifting_log_size, _ptr(out), _stream())
         return out
 
@@ -334,7 +341,7 @@ class CudaBackend:
         total = (1 << (lifting_log_size + 1)) - 1 if columns else 1
         layers = torch.empty((total, 8), dtype=torch.int32, device="cuda")
         tab = _ptr_table([c.data for c in columns])
-        logs = _u32_table([c.log_size for c in columns])
+        logs = _u32_table([c._log_size for c in columns])
         _lib.call("cs_merkle_commit", tab, logs, len(columns), lifting_log_size, _ptr(layers), _stream())
         return MerkleProverLifted(layers, lifting_log_size if columns else 0)
 
@@ -485,8 +492,7 @@ class CudaBackend:
         out = SecureColumnByCoords.uninitialized(1 << (lifting_log_size - log_blowup))
         tab = _ptr_table([c.data for a in accs for c in a.columns])
         logs = _u32_table([len(a).bit_length() - 1 for a in accs])
-        pts = np.ascontiguousarray(np.concatenate([np.concatenate([np.asarray(x, np.uint32), np.asarray(y, np.uint32)])
-                                                   for x, y in points]))
+        pts = np.array([w for point in points for coord in point for w in coord], np.uint32)
         fl = np.ascontiguousarray(np.asarray(first_linear, np.uint32).reshape(-1))
         _lib.call("cs_quotients_on_subdomain", tab, logs, len(accs), pts.ctypes.data, fl.ctypes.data,
                   lifting_log_size, log_blowup, _ptr_table([c.data for c in out.columns]), _stream())

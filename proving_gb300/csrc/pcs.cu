@@ -577,12 +577,15 @@ void fill_domain_tables(DomainTables& d, uint32_t half_init, uint32_t half_step)
       if ((idx >> b) & 1) r = cpoint_add(r, g.p[b]);
     return r;
   };
+  // T0[a] = init + a step, T1[a] = 2^9 a step, T2[a] = 2^18 a step, one addition per entry; the three
+  // chains side by side, since each waits for its last addition
+  cpoint step[3];
   for (uint32_t t = 0; t < 3; t++) {
-    // T0[a] = init + a step, T1[a] = 2^9 a step, T2[a] = 2^18 a step, one addition per entry
-    const cpoint step = point_at_host(((1u << (9 * t)) * half_step) & 0x7fffffffu);
+    step[t] = point_at_host(((1u << (9 * t)) * half_step) & 0x7fffffffu);
     d.t[t][0] = t == 0 ? point_at_host(half_init) : cpoint{1, 0};
-    for (uint32_t a = 1; a < 512; a++) d.t[t][a] = cpoint_add(d.t[t][a - 1], step);
   }
+  for (uint32_t a = 1; a < 512; a++)
+    for (uint32_t t = 0; t < 3; t++) d.t[t][a] = cpoint_add(d.t[t][a - 1], step[t]);
 }
 
 cs_status quotients_on_subdomain(const QuotientParams& q, uint32_t* const out[4], cudaStream_t st) {

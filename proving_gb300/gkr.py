@@ -593,24 +593,27 @@ def prove_batch_native(channel, input_layers) -> tuple[GkrBatchProof, GkrArtifac
     def take():
         nonlocal pos
         pos += 1
-        return int(w[pos - 1])
+        return w[pos - 1]
 
-    def felt():
+    def felts(n):
         nonlocal pos
-        pos += 4
-        return tuple(int(x) for x in w[pos - 4:pos])
+        first, pos = pos, pos + 4 * n
+        return [tuple(w[i:i + 4]) for i in range(first, pos, 4)]
 
     proof = GkrBatchProof()
     for _ in range(take()):
-        proof.sumcheck_proofs.append([[felt() for _ in range(take())] for _ in range(take())])
+        proof.sumcheck_proofs.append([felts(take()) for _ in range(take())])
     n_inst = take()
     for _ in range(n_inst):
-        proof.layer_masks_by_instance.append(
-            [GkrMask([(felt(), felt()) for _ in range(take())]) for _ in range(take())])
+        masks = []
+        for _ in range(take()):
+            values = felts(2 * take())
+            masks.append(GkrMask(list(zip(values[0::2], values[1::2]))))
+        proof.layer_masks_by_instance.append(masks)
     for _ in range(n_inst):
-        proof.output_claims_by_instance.append([felt() for _ in range(take())])
-    ood = [felt() for _ in range(take())]
-    claims = [[felt() for _ in range(take())] for _ in range(n_inst)]
+        proof.output_claims_by_instance.append(felts(take()))
+    ood = felts(take())
+    claims = [felts(take()) for _ in range(n_inst)]
     n_vars = [take() for _ in range(n_inst)]
     channel.digest = struct.pack("<8I", *snap[:8])
     channel.n_draws = snap[8]
