@@ -15,6 +15,7 @@
 //    barycentric derivative term is 4^(l-1) * prod_{k<l} pi^(k-1)(x_i).
 //  * sums of M31 products are accumulated in 64 bits and reduced once.
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -328,6 +329,146 @@ __global__ void __launch_bounds__(kBaryThreads, 3) bary_partial_kernel(const Bar
   }
 }
 
+// The same sums on the tensor cores, for long columns: out[c][k] = sum_r x_c[r] w_k[r] is a contraction
+// over the rows, and with both factors split into four bytes every product of two bytes is exact in half
+// precision and sums of up to 256 of them (255^2 each, below 2^24) in the single-precision
+// accumulators, which are then emptied into 64-bit sums. m16n8k16: K is 16 rows, N the
+// (coordinate, byte) pairs of the weights (two tiles), M the (column, byte) pairs of eight columns (two
+// tiles: bytes 0, 1 and 2, 3), mapped so that a lane's fragments come from words it loads itself: lane
+// (g, q) reads rows 4 q .. 4 q + 3 of column g and of the weights' coordinates g / 4 and 2 + g / 4. A byte
+// becomes a half as 0x6400 | b (1024 + b) less 1024. About 9 instructions per 32 (row, column)
+// pairs against 39 for the multiply-adds. The columns come in tiles of 512 rows by cp.async, two
+// tiles deep: read from global memory by the lanes themselves, 64 bytes of a column at a time, the tens of
+// thousands of streams in flight cost DRAM more than the arithmetic saved. Bound: HBM.
+// 64 columns of 2^20: 82.5 -> 50.2 us (69.9 with the lanes' own loads); the mixed proof's 26 sets 3.99 ->
+// 2.44 ms (4.94).
+constexpr uint32_t kBaryMmaMinLog = 12;
+constexpr int kBaryMmaCols = 16;           // columns per block (two groups of eight)
+constexpr uint32_t kBaryTile = 512;        // rows a tile, 64 a warp
+constexpr uint32_t kBaryStream = kBaryTile + 16;  // words: 64 bytes of padding keep eight columns on distinct banks
+constexpr uint32_t kBaryStreams = kBaryMmaCols + 4;
+constexpr uint32_t kBarySmem = 2 * kBaryStreams * kBaryStream * sizeof(uint32_t);
+
+// Two half-precision integers from the bytes of t that `sel` names (0x6400 | byte, less 1024).
+__device__ __forceinline__ uint32_t byte_halves(uint32_t t, uint32_t sel) {
+  const uint32_t h = __byte_perm(t, 0x64646464u, sel);
+  uint32_t r;
+  asm("add.f16x2 %0, %1, %2;" : "=r"(r) : "r"(h), "r"(0xe400e400u));
+  return r;
+}
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// One tile of the block's columns and the weights into shared memory.
+__device__ __forceinline__ void load_bary_tile(const uint32_t* const* ptr, uint32_t row, uint32_t* stage) {
+#pragma unroll
+  for (uint32_t k = 0; k < kBaryStreams * kBaryTile / 4 / kBaryThreads; k++) {
+    const uint32_t i = threadIdx.x + k * kBaryThreads;  // 16-byte word of the tile
+    const uint32_t stream = i / (kBaryTile / 4), word = i % (kBaryTile / 4);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(
+                     stage + stream * kBaryStream + 4 * word)),
+                 "l"(ptr[stream] + row + 4 * word));
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kBaryThreads, 2) bary_mma_kernel(const __grid_constant__ BaryColumns cols, uint32_t nb,
+                                                                   uint32_t n, CSoA w, unsigned long long* partial) {
+  extern __shared__ __align__(16) uint32_t tiles[];
+  __shared__ uint32_t sh[kBaryThreads / 32][kBaryMmaCols][4];
+  __shared__ const uint32_t* ptr[kBaryStreams];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const uint32_t c0 = blockIdx.y * kBaryMmaCols;
+  if (threadIdx.x < kBaryStreams)
+    ptr[threadIdx.x] = threadIdx.x < kBaryMmaCols ? cols.ptr[min(c0 + threadIdx.x, nb - 1)] : w.c[threadIdx.x - kBaryMmaCols];
+  __syncthreads();
+  const uint32_t bsel = (g & 3) | ((4 + (g & 3)) << 4);  // byte g & 3 of two words
+  // a lane has, of column g of each group, every byte i of the column and bytes 2 (q & 1) and + 1 of the
+  // weights' coordinates q / 2 and 2 + q / 2; byte i times byte j counts 2^(8 (i + j)) = 2^(8 (i + j) mod 31)
+  float acc[2][2][2][4];  // [group][bytes 0, 1 or 2, 3][coordinates 0, 1 or 2, 3][+ row 8][+ column 1]
+  uint64_t sum[2][2] = {{0, 0}, {0, 0}};  // [group][coordinates]
+#pragma unroll
+  for (int i = 0; i < 32; i++) (&acc[0][0][0][0])[i] = 0;
+  const uint32_t odd = q & 1;
+  const uint32_t n_tiles = n / kBaryTile;
+  uint32_t filled = 0;  // tiles summed since the last emptying: 64 rows each
+  load_bary_tile(ptr, blockIdx.x * kBaryTile, tiles);
+#pragma unroll 1
+  for (uint32_t tile = blockIdx.x, stage = 0; tile < n_tiles; tile += gridDim.x, stage ^= 1) {
+    if (tile + gridDim.x < n_tiles) {
+      load_bary_tile(ptr, (tile + gridDim.x) * kBaryTile, tiles + (stage ^ 1) * kBaryStreams * kBaryStream);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const uint32_t* t0 = tiles + stage * kBaryStreams * kBaryStream + warp * 64 + 4 * q;
+#pragma unroll
+    for (uint32_t step = 0; step < 64; step += 16) {
+      const auto at = [&](uint32_t stream) { return *reinterpret_cast<const uint4*>(t0 + stream * kBaryStream + step); };
+      uint32_t b[2][2];
+#pragma unroll
+      for (int t = 0; t < 2; t++) {
+        const uint4 v = at(kBaryMmaCols + 2 * t + (g >> 2));
+        b[t][0] = byte_halves(__byte_perm(v.x, v.y, bsel), 0x4140);
+        b[t][1] = byte_halves(__byte_perm(v.z, v.w, bsel), 0x4140);
+      }
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        const uint4 v = at(8 * c + g);
+        // bytes 0, 1 (lo) and 2, 3 (hi) of two rows, interleaved
+        const uint32_t lo0 = __byte_perm(v.x, v.y, 0x5140), hi0 = __byte_perm(v.x, v.y, 0x7362);
+        const uint32_t lo1 = __byte_perm(v.z, v.w, 0x5140), hi1 = __byte_perm(v.z, v.w, 0x7362);
+        const uint32_t a0[4] = {byte_halves(lo0, 0x4140), byte_halves(lo0, 0x4342), byte_halves(lo1, 0x4140),
+                                byte_halves(lo1, 0x4342)};
+        const uint32_t a1[4] = {byte_halves(hi0, 0x4140), byte_halves(hi0, 0x4342), byte_halves(hi1, 0x4140),
+                                byte_halves(hi1, 0x4342)};
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+          mma_f16(acc[c][0][t], a0, b[t]);
+          mma_f16(acc[c][1][t], a1, b[t]);
+        }
+      }
+    }
+    __syncthreads();  // the stage is free again
+    if (++filled < 4 && tile + gridDim.x < n_tiles) continue;
+    filled = 0;
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const int i = 2 * h + (e >> 1), j = e & 1;
+            const uint32_t weight = odd ? 1u << (8 * (i + j + 2) % 31) : 1u << (8 * (i + j) % 31);
+            sum[c][t] += (uint64_t)__float2uint_rn(acc[c][h][t][e]) * weight;
+            acc[c][h][t][e] = 0;
+          }
+  }
+#pragma unroll
+  for (int c = 0; c < 2; c++)
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+      uint32_t v = m31_reduce64(sum[c][t]);
+      v = m31_add(v, __shfl_xor_sync(0xffffffffu, v, 1));
+      if (!odd) sh[warp][8 * c + g][2 * t + (q >> 1)] = v;
+    }
+  __syncthreads();
+  const uint32_t t = threadIdx.x;
+  if (t < 4 * kBaryMmaCols && c0 + (t >> 2) < nb) {
+    uint64_t total = 0;
+#pragma unroll
+    for (int k = 0; k < kBaryThreads / 32; k++) total += sh[k][t >> 2][t & 3];
+    partial[((size_t)c0 * 4 + t) * gridDim.x + blockIdx.x] = total;
+  }
+}
+
 // One warp per (column, coordinate): its row of per-chunk partial sums, strided over the lanes.
 __global__ void bary_final_kernel(const unsigned long long* partial, uint32_t n_chunks, uint32_t nb, uint32_t* out) {
   const uint32_t row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -610,6 +751,22 @@ cs_status quotients_on_subdomain(const QuotientParams& q, uint32_t* const out[4]
 
 using namespace cs;
 
+// The tensor-core kernel's shared memory limit, raised once per device.
+static cudaError_t allow_bary_smem() {
+  static std::mutex mu;
+  static bool done[kMaxDevices] = {false};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!done[dev]) {
+    e = cudaFuncSetAttribute(bary_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBarySmem);
+    done[dev] = e == cudaSuccess;
+  }
+  return e;
+}
+
 static cs_status check4(const uint32_t* const p[4], const char* what) {
   CS_CHECK_ARG(p != nullptr, "%s: null coordinate table", what);
   for (int k = 0; k < 4; k++) CS_CHECK_ARG(p[k] != nullptr, "%s: coordinate %d is null", what, k);
@@ -748,12 +905,27 @@ extern "C" cs_status cs_barycentric_eval(const uint32_t* const* h_cols, uint32_t
       CS_CHECK_ARG(h_cols[b0 + i] != nullptr, "barycentric_eval: column %u is null", b0 + i);
       cols.ptr[i] = h_cols[b0 + i];
     }
-    const uint32_t n_chunks = ((1u << log_size) + kBaryChunk - 1) / kBaryChunk;
+    const uint32_t n = 1u << log_size;
+    bool mma = log_size >= kBaryMmaMinLog;
+    for (int k = 0; k < 4; k++) mma = mma && aligned16(w.c[k]);
+    for (uint32_t i = 0; i < nb; i++) mma = mma && aligned16(cols.ptr[i]);
+    const uint32_t groups = (nb + kBaryMmaCols - 1) / kBaryMmaCols;
+    // tensor cores: the two blocks an SM that fit share the tiles of every group
+    const uint32_t n_chunks = mma ? std::min(n / kBaryTile, std::max(1u, 2 * 152 / groups))
+                                  : (n + kBaryChunk - 1) / kBaryChunk;
     cudaStream_t st = to_stream(stream);
     unsigned long long* partial = nullptr;
     CS_CUDA(stream_alloc(reinterpret_cast<void**>(&partial), sizeof(unsigned long long) * 4 * nb * n_chunks, st));
-    bary_partial_kernel<<<dim3(n_chunks, (nb + kBaryGroup - 1) / kBaryGroup), kBaryThreads, 0, st>>>(
-        cols, nb, log_size, w, partial);
+    if (mma) {
+      cudaError_t attr = allow_bary_smem();
+      if (attr != cudaSuccess) {
+        cudaFreeAsync(partial, st);
+        return from_cuda(attr, "barycentric_eval");
+      }
+      bary_mma_kernel<<<dim3(n_chunks, groups), kBaryThreads, kBarySmem, st>>>(cols, nb, n, w, partial);
+    } else
+      bary_partial_kernel<<<dim3(n_chunks, (nb + kBaryGroup - 1) / kBaryGroup), kBaryThreads, 0, st>>>(
+          cols, nb, log_size, w, partial);
     note_launch();
     bary_final_kernel<<<(4 * nb + 7) / 8, 256, 0, st>>>(partial, n_chunks, nb, d_out + 4 * b0);
     note_launch();
