@@ -27,7 +27,7 @@
 //      the claimed sum, kept in device memory;
 //   3. outputs: per pair of mirror tiles (m, ~m), the natural prefixes of both
 //      and then every output of both.
-// Columns of at most 2^9 rows are done by one block in the first launch.
+// Columns of at most 2^9 rows are done by one block each, in a launch of their own.
 #include <algorithm>
 #include <vector>
 
@@ -43,13 +43,14 @@ namespace {
 constexpr uint32_t kSumBatch = 48;  // columns per launch (their pointers travel as kernel parameters)
 constexpr uint32_t kSmallLog = 9;   // columns up to 2^9 rows: one block each
 constexpr uint32_t kThreads = 1024;
+constexpr uint32_t kTileThreads = 256;
 
 struct SumBatch {
   const uint32_t* values[kSumBatch];  // the looked-up values (fractions 1 / (z - v)), or null:
                                       // the fractions are already in `out`
   uint32_t* out[kSumBatch][4];
   uint32_t log_size[kSumBatch];
-  uint32_t tile0[kSumBatch + 1];  // first launch-1 block of each column (one per tile; one if small)
+  uint32_t tile0[kSumBatch + 1];  // first launch-1 block of each column (one per tile; none if small)
   uint32_t pair0[kSumBatch + 1];  // first launch-3 block of each column (none if small)
   uint32_t run0[kSumBatch];       // first run total of each column in `runs` (4 words each)
   uint32_t hoff0[kSumBatch];      // the column's 32 segment offsets in `runs`
@@ -141,6 +142,22 @@ __device__ __forceinline__ void warp_scan4(uint32_t x[4]) {
   }
 }
 
+// The warp's sum of r[0..3] (each below P): coordinate lane >> 3 in lanes 0, 8, 16, 24. The first two
+// steps halve the coordinates a lane keeps: 6 shuffles instead of 20.
+__device__ __forceinline__ uint32_t warp_sum4(const uint32_t r[4], uint32_t lane) {
+  const bool hi = (lane >> 4) & 1;  // keeps coordinates 2, 3
+  uint32_t k0 = hi ? r[2] : r[0], k1 = hi ? r[3] : r[1];
+  const uint32_t s0 = hi ? r[0] : r[2], s1 = hi ? r[1] : r[3];
+  k0 = m31_add(k0, __shfl_xor_sync(0xffffffffu, s0, 16));
+  k1 = m31_add(k1, __shfl_xor_sync(0xffffffffu, s1, 16));
+  const bool odd = (lane >> 3) & 1;  // keeps the second of its pair
+  uint32_t v = odd ? k1 : k0;
+  v = m31_add(v, __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 8));
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v = m31_add(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
 // A column of at most 2^9 rows, all in one block (at least 2^9 threads).
 __device__ void small_column(const SumBatch& b, uint32_t col, uint32_t* flat, uint32_t (*sh)[32]) {
   const uint32_t log_n = b.log_size[col], n = 1u << log_n, t = threadIdx.x;
@@ -174,86 +191,94 @@ __device__ void small_column(const SumBatch& b, uint32_t col, uint32_t* flat, ui
   if (t < 4) b.claimed[4 * col + t] = t == 0 ? total.a.a : t == 1 ? total.a.b : t == 2 ? total.b.a : total.b.b;
 }
 
-// 1 / (z - v0) and 1 / (z - v1) with one M31 inversion (Montgomery's trick on the norms): for
-// x = a + b u, 1 / x = (a - b u) / (a^2 - (2 + i) b^2), and 1 / d = conj(d) / |d|^2 for d in CM31.
-__device__ __forceinline__ void fraction_pair(const qm31& z, uint32_t v0, uint32_t v1, qm31& f0, qm31& f1) {
-  const qm31 x0 = qm31_sub(z, qm31_make(v0, 0, 0, 0)), x1 = qm31_sub(z, qm31_make(v1, 0, 0, 0));
-  const auto denom = [](const qm31& x) {
-    const cm31 b2 = cm31_mul(x.b, x.b);
-    const cm31 ib2 = {m31_neg(b2.b), b2.a};
-    return cm31_sub(cm31_mul(x.a, x.a), cm31_add(cm31_add(b2, b2), ib2));
-  };
-  const cm31 d0 = denom(x0), d1 = denom(x1);
-  const uint32_t n0 = m31_add(m31_sqr(d0.a), m31_sqr(d0.b)), n1 = m31_add(m31_sqr(d1.a), m31_sqr(d1.b));
-  const uint32_t prod = m31_mul(n0, n1);
-  uint32_t i0, i1;
-  if (prod != 0) {
-    const uint32_t inv = m31_inv(prod);
-    i0 = m31_mul(inv, n1);
-    i1 = m31_mul(inv, n0);
-  } else {  // z = v for one of them: each inverted alone (the inverse of 0 taken as 0, as in qm31_inv)
-    i0 = m31_inv(n0);
-    i1 = m31_inv(n1);
+// 1 / (z - v) for kQuad values with one M31 inversion (Montgomery's trick on the norms): for
+// x = a + b u, 1 / x = (a - b u) / (a^2 - (2 + i) b^2), and 1 / d = conj(d) / |d|^2 for d in CM31. With
+// a = t + z1 i, t = z0 - v, the CM31 norm is (t^2 - re0) + (im1 t - im0) i for constants of z alone.
+constexpr int kQuad = 4;
+__device__ __forceinline__ void fraction_quad(const qm31& z, const uint32_t (&v)[kQuad], qm31 (&f)[kQuad]) {
+  const cm31 b2 = cm31_mul(z.b, z.b);  // (2 + i)(p + q i) = (2 p - q) + (p + 2 q) i
+  const uint32_t re0 = m31_add(m31_sqr(z.a.b), m31_sub(m31_add(b2.a, b2.a), b2.b));
+  const uint32_t im0 = m31_add(b2.a, m31_add(b2.b, b2.b)), im1 = m31_add(z.a.b, z.a.b);
+  uint32_t t[kQuad], norm[kQuad], pre[kQuad], acc = 1;
+  cm31 d[kQuad];
+#pragma unroll
+  for (int k = 0; k < kQuad; k++) {
+    t[k] = m31_sub(z.a.a, v[k]);
+    d[k] = {m31_sub(m31_sqr(t[k]), re0), m31_sub(m31_mul(t[k], im1), im0)};
+    norm[k] = m31_reduce64((uint64_t)d[k].a * d[k].a + (uint64_t)d[k].b * d[k].b);
+    pre[k] = acc;
+    acc = m31_mul(acc, norm[k] == 0 ? 1u : norm[k]);  // z = v: the inverse of 0 is taken as 0, as in qm31_inv
   }
-  const cm31 di0 = {m31_mul(d0.a, i0), m31_mul(m31_neg(d0.b), i0)};
-  const cm31 di1 = {m31_mul(d1.a, i1), m31_mul(m31_neg(d1.b), i1)};
-  f0 = {cm31_mul(x0.a, di0), cm31_mul(cm31_neg(x0.b), di0)};
-  f1 = {cm31_mul(x1.a, di1), cm31_mul(cm31_neg(x1.b), di1)};
+  acc = m31_inv(acc);
+#pragma unroll
+  for (int k = kQuad - 1; k >= 0; k--) {
+    const uint32_t inv = norm[k] == 0 ? 0 : m31_mul(acc, pre[k]);
+    acc = m31_mul(acc, norm[k] == 0 ? 1u : norm[k]);
+    const cm31 di = {m31_mul(d[k].a, inv), m31_neg(m31_mul(d[k].b, inv))};
+    f[k] = {cm31_mul(cm31{t[k], z.a.b}, di), cm31_neg(cm31_mul(z.b, di))};
+  }
 }
 
-// Launch 1 (512 threads): per tile m of a column of 2^10 or more rows, thread (w, t) (w < 16) takes
-// the storage positions (rev5(lo) << (l - 5)) | (rev(m) << 5) | t for lo = w and w + 16, i.e.
-// natural (h = rev5(t), m, lo); their two fractions share one M31 inversion.
-__global__ void __launch_bounds__(kThreads / 2) runs_kernel(const SumBatch b) {
+// Launch 1 (256 threads): per tile m of a column of 2^10 or more rows,
+// thread (w, t) (w < 8) takes the storage positions (rev5(lo) << (l - 5)) | (rev(m) << 5) | t for
+// lo = w + 8 q, q < 4, i.e. natural (h = rev5(t), m, lo); its four fractions share one M31 inversion and
+// its four loads are in flight together. Bound: the inversion's chain and HBM (4 bytes read, 16 written a
+// row). One position a thread, 1,024 threads and an inversion each took 1.75 ms over the 120 columns (2^10
+// to 2^22 rows) of a mixed proof; this takes 1.13 ms. Columns of 2^9 rows or fewer have a kernel of their
+// own so that its registers and shared memory are not this one's.
+__global__ void __launch_bounds__(kTileThreads) runs_kernel(const SumBatch b) {
   __shared__ uint32_t tile[4][32][33];
-  __shared__ uint32_t sh[4][32];
   const uint32_t col = block_column(b.tile0, b.n_cols, blockIdx.x);
   const uint32_t log_n = b.log_size[col];
-  if (log_n <= kSmallLog) {
-    small_column(b, col, &tile[0][0][0], sh);
-    return;
-  }
   const uint32_t mb = log_n - 10, m = blockIdx.x - b.tile0[col];
   const uint32_t w = threadIdx.x >> 5, t = threadIdx.x & 31, h = rev5(t);
   const uint32_t mid = (rev_bits(m, mb) << 5) | t;
-  const uint32_t p0 = (rev5(w) << (log_n - 5)) | mid, p1 = (rev5(w + 16) << (log_n - 5)) | mid;
-  qm31 g[2];
+  uint32_t p[kQuad];
+  qm31 g[kQuad];
+#pragma unroll
+  for (int q = 0; q < kQuad; q++) p[q] = (rev5(w + 8 * q) << (log_n - 5)) | mid;
   if (b.values[col] != nullptr) {
-    fraction_pair(b.z, b.values[col][p0], b.values[col][p1], g[0], g[1]);
-    store4(b, col, p0, g[0]);
-    store4(b, col, p1, g[1]);
+    uint32_t v[kQuad];
+#pragma unroll
+    for (int q = 0; q < kQuad; q++) v[q] = b.values[col][p[q]];
+    fraction_quad(b.z, v, g);
+#pragma unroll
+    for (int q = 0; q < kQuad; q++) store4(b, col, p[q], g[q]);
   } else {
-    g[0] = load_fraction(b, col, p0);
-    g[1] = load_fraction(b, col, p1);
+#pragma unroll
+    for (int q = 0; q < kQuad; q++) g[q] = load_fraction(b, col, p[q]);
   }
 #pragma unroll
-  for (int q = 0; q < 2; q++) {
-    const uint32_t lo = w + 16 * q;
+  for (int q = 0; q < kQuad; q++) {
+    const uint32_t lo = w + 8 * q;
     tile[0][lo][h] = g[q].a.a;
     tile[1][lo][h] = g[q].a.b;
     tile[2][lo][h] = g[q].b.a;
     tile[3][lo][h] = g[q].b.b;
   }
   __syncthreads();
-  // warp w sums natural runs (h' = w and w + 16, m): lanes are lo
+  // warp w sums natural runs (h' = w + 8 q, m): lanes are lo
 #pragma unroll
-  for (int q = 0; q < 2; q++) {
-    const uint32_t hh = w + 16 * q;
+  for (int q = 0; q < kQuad; q++) {
+    const uint32_t hh = w + 8 * q;
     uint32_t x[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) x[k] = tile[k][t][hh];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) x[k] = m31_add(x[k], __shfl_xor_sync(0xffffffffu, x[k], o));
-    }
-    if (t < 4) b.runs[4 * (b.run0[col] + ((hh << mb) | m)) + t] = x[t];
+    const uint32_t v = warp_sum4(x, t);  // coordinate t / 8, in lanes 0, 8, 16, 24
+    if ((t & 7) == 0) b.runs[4 * (b.run0[col] + ((hh << mb) | m)) + (t >> 3)] = v;
   }
+}
+
+// Columns of at most 2^9 rows: one block each.
+__global__ void __launch_bounds__(kThreads / 2) small_kernel(const SumBatch b) {
+  __shared__ uint32_t flat[4 * 512];
+  __shared__ uint32_t sh[4][32];
+  if (b.log_size[blockIdx.x] <= kSmallLog) small_column(b, blockIdx.x, flat, sh);
 }
 
 // Launch 2: one block per column of 2^10 or more rows. The natural runs (h, m) are ordered h-major,
 // so warp h owns the contiguous runs [h 2^mb, (h + 1) 2^mb): it turns them into exclusive offsets
-// within its segment (coalesced, 32 runs per step), and the block turns the 32 segment totals into
+// within its segment (coalesced, 128 runs per step, their loads in flight together), and the block turns the 32 segment totals into
 // the segment offsets `hoff` (added by launch 3); the grand total is the claimed sum.
 __global__ void __launch_bounds__(kThreads) run_offsets_kernel(const SumBatch b) {
   __shared__ uint32_t seg_total[4][32];
@@ -264,16 +289,26 @@ __global__ void __launch_bounds__(kThreads) run_offsets_kernel(const SumBatch b)
   const uint32_t h = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint4* r = reinterpret_cast<uint4*>(b.runs) + b.run0[col] + (size_t)h * seg;
   uint32_t carry[4] = {0, 0, 0, 0};
-  for (uint32_t base = 0; base < seg; base += 32) {
-    const bool live = base + lane < seg;
-    const uint4 v = live ? r[base + lane] : make_uint4(0, 0, 0, 0);
-    uint32_t x[4] = {v.x, v.y, v.z, v.w};
-    warp_scan4(x);
-    if (live)
-      r[base + lane] = make_uint4(m31_add(m31_sub(x[0], v.x), carry[0]), m31_add(m31_sub(x[1], v.y), carry[1]),
-                                  m31_add(m31_sub(x[2], v.z), carry[2]), m31_add(m31_sub(x[3], v.w), carry[3]));
+  for (uint32_t base = 0; base < seg; base += 32 * kQuad) {
+    uint4 v[kQuad];
+    uint32_t x[kQuad][4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) carry[k] = m31_add(carry[k], __shfl_sync(0xffffffffu, x[k], 31));
+    for (int q = 0; q < kQuad; q++) {
+      const uint32_t i = base + 32 * q + lane;
+      v[q] = i < seg ? r[i] : make_uint4(0, 0, 0, 0);
+      x[q][0] = v[q].x, x[q][1] = v[q].y, x[q][2] = v[q].z, x[q][3] = v[q].w;
+    }
+#pragma unroll
+    for (int q = 0; q < kQuad; q++) warp_scan4(x[q]);
+#pragma unroll
+    for (int q = 0; q < kQuad; q++) {
+      const uint32_t i = base + 32 * q + lane;
+      if (i < seg)
+        r[i] = make_uint4(m31_add(m31_sub(x[q][0], v[q].x), carry[0]), m31_add(m31_sub(x[q][1], v[q].y), carry[1]),
+                          m31_add(m31_sub(x[q][2], v[q].z), carry[2]), m31_add(m31_sub(x[q][3], v[q].w), carry[3]));
+#pragma unroll
+      for (int k = 0; k < 4; k++) carry[k] = m31_add(carry[k], __shfl_sync(0xffffffffu, x[q][k], 31));
+    }
   }
   if (lane == 0) {
 #pragma unroll
@@ -296,52 +331,85 @@ __global__ void __launch_bounds__(kThreads) run_offsets_kernel(const SumBatch b)
   }
 }
 
-// Launch 3: per mirror pair of tiles (m, m' = ~m) of a column of 2^10 or more rows.
-__global__ void __launch_bounds__(kThreads) outputs_kernel(const SumBatch b) {
+// Launch 3 (256 threads): per mirror pair of tiles (m, m' = ~m) of a column of 2^10 or more rows; a thread
+// has four elements of each tile, whose loads are in flight together. Bound: HBM (16 bytes read, 16 written
+// a row; the second read of a fraction hits L1 or L2) and the scans' shuffles. With 1,024 threads of one
+// element the three waves of a block left the memory idle in between: 2.17 ms for the same 120 columns,
+// 1.49 ms here.
+__global__ void __launch_bounds__(kTileThreads) outputs_kernel(const SumBatch b) {
   __shared__ uint32_t tiles[2][4][32][33];
   const uint32_t col = block_column(b.pair0, b.n_cols, blockIdx.x);
-  const uint32_t log_n = b.log_size[col];
+  const uint32_t log_n = b.log_size[col], n = 1u << log_n;
   const uint32_t mb = log_n - 10;
   const uint32_t m = blockIdx.x - b.pair0[col], mm = ((1u << mb) - 1) - m;
   const uint32_t n_tiles = m == mm ? 1 : 2;
   const uint32_t w = threadIdx.x >> 5, t = threadIdx.x & 31, h = rev5(t);
   const uint32_t ms[2] = {m, mm};
-  qm31 g[2];
-  uint32_t pos[2];
-  for (uint32_t q = 0; q < n_tiles; q++) {
-    pos[q] = (rev5(w) << (log_n - 5)) | (rev_bits(ms[q], mb) << 5) | t;
-    const uint32_t p = pos[q];
-    g[q] = qm31_make(b.out[col][0][p], b.out[col][1][p], b.out[col][2][p], b.out[col][3][p]);
-    tiles[q][0][w][h] = g[q].a.a;
-    tiles[q][1][w][h] = g[q].a.b;
-    tiles[q][2][w][h] = g[q].b.a;
-    tiles[q][3][w][h] = g[q].b.b;
+  uint32_t* const out[4] = {b.out[col][0], b.out[col][1], b.out[col][2], b.out[col][3]};
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    if ((uint32_t)q >= n_tiles) break;
+    const uint32_t mid = (rev_bits(ms[q], mb) << 5) | t;
+    uint32_t g[kQuad][4];
+#pragma unroll
+    for (int j = 0; j < kQuad; j++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) g[j][k] = out[k][(rev5(w + 8 * j) << (log_n - 5)) | mid];
+#pragma unroll
+    for (int j = 0; j < kQuad; j++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) tiles[q][k][w + 8 * j][h] = g[j][k];
   }
   __syncthreads();
-  const uint32_t* r = b.runs + 4 * (size_t)b.run0[col];
-  const uint32_t* hoff = b.runs + 4 * (size_t)b.hoff0[col] + 4 * w;  // segment h = w
-  for (uint32_t q = 0; q < n_tiles; q++) {
-    // warp w: natural run (h = w, ms[q]); lanes are lo
-    uint32_t x[4];
+  const uint4* r = reinterpret_cast<const uint4*>(b.runs) + b.run0[col];
+  const uint4* hoff = reinterpret_cast<const uint4*>(b.runs) + b.hoff0[col];
 #pragma unroll
-    for (int k = 0; k < 4; k++) x[k] = tiles[q][k][t][w];
-    warp_scan4(x);
-    const uint32_t run = (w << mb) | ms[q];
+  for (int q = 0; q < 2; q++) {
+    if ((uint32_t)q >= n_tiles) break;
 #pragma unroll
-    for (int k = 0; k < 4; k++) tiles[q][k][t][w] = m31_add(m31_add(x[k], r[4 * run + k]), hoff[k]);
+    for (int j = 0; j < kQuad; j++) {
+      // natural run (hh, ms[q]); lanes are lo
+      const uint32_t hh = w + 8 * j;
+      uint32_t x[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = tiles[q][k][t][hh];
+      const uint4 run = r[(hh << mb) | ms[q]], seg = hoff[hh];
+      warp_scan4(x);
+      tiles[q][0][t][hh] = m31_add(x[0], m31_add(run.x, seg.x));
+      tiles[q][1][t][hh] = m31_add(x[1], m31_add(run.y, seg.y));
+      tiles[q][2][t][hh] = m31_add(x[2], m31_add(run.z, seg.z));
+      tiles[q][3][t][hh] = m31_add(x[3], m31_add(run.w, seg.w));
+    }
   }
   __syncthreads();
-  const qm31 total = qm31_make(b.claimed[4 * col], b.claimed[4 * col + 1], b.claimed[4 * col + 2],
-                               b.claimed[4 * col + 3]);
-  for (uint32_t q = 0; q < n_tiles; q++) {
-    // element (h, ms[q], lo = w); its mirror (31 - h, ms[1 - q], 31 - w) is in the other tile
-    // (the same one when m = m')
-    const uint32_t o = n_tiles == 1 ? 0 : 1 - q;
-    const qm31 qp = qm31_make(tiles[q][0][w][h], tiles[q][1][w][h], tiles[q][2][w][h], tiles[q][3][w][h]);
-    const qm31 qm = qm31_make(tiles[o][0][31 - w][31 - h], tiles[o][1][31 - w][31 - h], tiles[o][2][31 - w][31 - h],
-                              tiles[o][3][31 - w][31 - h]);
-    const uint32_t c = (h << (log_n - 5)) | (ms[q] << 5) | w;
-    store4(b, col, pos[q], running_value(c, log_n, qp, qm, g[q], total));
+  uint32_t total[4], shift[4];  // shift = total / n, 1 / n = 2^(31 - log_n) in M31
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    total[k] = b.claimed[4 * col + k];
+    shift[k] = m31_mul_pow2(total[k], 31 - log_n);
+  }
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    if ((uint32_t)q >= n_tiles) break;
+    // element (h, ms[q], lo); its mirror (31 - h, ms[1 - q], 31 - lo) is in the other tile (the same one
+    // when m = m'). The fraction is the difference of two prefixes of its run, the first one's less the
+    // run's offset: read it again instead.
+    const int o = n_tiles == 1 ? 0 : 1 - q;
+    const uint32_t mid = (rev_bits(ms[q], mb) << 5) | t;
+#pragma unroll
+    for (int j = 0; j < kQuad; j++) {
+      const uint32_t lo = w + 8 * j, p = (rev5(lo) << (log_n - 5)) | mid;
+      const uint32_t c = (h << (log_n - 5)) | (ms[q] << 5) | lo;
+      const bool first_half = c < (n >> 1);
+      const uint32_t steps = (first_half ? 2 * c : 2 * n - 1 - 2 * c) + 1;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t qp = tiles[q][k][lo][h], qm = tiles[o][k][31 - lo][31 - h];
+        const uint32_t v = first_half ? m31_sub(m31_add(qp, total[k]), qm)
+                                      : m31_add(m31_sub(m31_add(qm, total[k]), qp), out[k][p]);
+        out[k][p] = m31_sub(v, m31_mul(shift[k], steps));
+      }
+    }
   }
 }
 
@@ -362,6 +430,7 @@ cs_status scan_columns(const uint32_t* const* values, const Q4* outs, const uint
     b.claimed = d_claimed + 4 * b0;
     b.runs = runs;
     uint32_t tiles = 0, pairs = 0;
+    bool small = false;
     for (uint32_t i = 0; i < b.n_cols; i++) {
       const uint32_t l = log_sizes[b0 + i];
       b.values[i] = values != nullptr ? values[b0 + i] : nullptr;
@@ -372,7 +441,7 @@ cs_status scan_columns(const uint32_t* const* values, const Q4* outs, const uint
       b.run0[i] = (uint32_t)run_base;
       b.hoff0[i] = 0;
       if (l <= kSmallLog) {
-        tiles += 1;
+        small = true;
       } else {
         tiles += 1u << (l - 10);
         pairs += l == 10 ? 1 : 1u << (l - 11);
@@ -382,12 +451,16 @@ cs_status scan_columns(const uint32_t* const* values, const Q4* outs, const uint
     }
     b.tile0[b.n_cols] = tiles;
     b.pair0[b.n_cols] = pairs;
-    runs_kernel<<<tiles, kThreads / 2, 0, st>>>(b);
-    note_launch();
+    if (small) {
+      small_kernel<<<b.n_cols, kThreads / 2, 0, st>>>(b);
+      note_launch();
+    }
     if (pairs > 0) {
+      runs_kernel<<<tiles, kTileThreads, 0, st>>>(b);
+      note_launch();
       run_offsets_kernel<<<b.n_cols, kThreads, 0, st>>>(b);
       note_launch();
-      outputs_kernel<<<pairs, kThreads, 0, st>>>(b);
+      outputs_kernel<<<pairs, kTileThreads, 0, st>>>(b);
       note_launch();
     }
     cudaError_t e = cudaGetLastError();
