@@ -581,6 +581,106 @@ __global__ void numerators_kernel(const NumeratorTerms terms, uint32_t rows, SoA
   }
 }
 
+// The same rows on the tensor cores (see bary_mma_kernel for the exactness of byte products): out[r][k] =
+// sum_t col_t[r] c_t[k] is a contraction over the terms. K is the four bytes x_i of four columns' words (16),
+// N the four bytes of the four coordinates of c_t 2^(8 i) mod P (16, two tiles), so the sums over i come
+// out of the products themselves; M is the rows. A lane's fragment is the words it loads: lane (g, q) reads
+// 16 bytes, rows 4 g .. 4 g + 3, of column q of the step, 128 bytes of each column a warp, and gets
+// coordinate q of the same rows back, so that neither side goes through shared memory or shuffles. A byte b
+// is used as the half 0x00bb = b 2^-24; the accumulators are exact multiples of 2^-24 below 1 for up
+// to 64 columns and are then emptied into 64-bit sums. Bound: HBM (8 loads of 512 bytes a warp, 16 warps an
+// SM in flight; two steps prefetched instead of four at once, 24 warps an SM or both were 5% to 27% slower).
+// 150 terms of 2^22 rows: 549 us by multiply-adds, 423 here (6.2 TB/s); 64 of 2^20: 65 and 62.
+constexpr int kNumThreads = 256;
+constexpr uint32_t kNumRows = 64;  // rows a warp: two loads a step for one set of coefficient fragments
+constexpr uint32_t kNumUnroll = 4;
+// With fewer terms a warp has too little in flight per pass over its rows: 24 terms of 2^20 rows take 33.4 us
+// here against 30.7 by multiply-adds, 26 of 2^22 101 against 115.
+constexpr uint32_t kNumMmaMinTerms = 25;
+
+__global__ void __launch_bounds__(kNumThreads, 2) numerators_mma_kernel(const __grid_constant__ NumeratorTerms terms,
+                                                                        uint32_t rows, const __grid_constant__ SoA out,
+                                                                        bool accumulate) {
+  __shared__ uint4 frag[kMaxTerms / 4][32];
+  __shared__ const uint32_t* ptr[kMaxTerms];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const uint32_t steps = (terms.n + 4 * kNumUnroll - 1) / (4 * kNumUnroll) * kNumUnroll;
+  for (uint32_t i = threadIdx.x; i < steps * 32; i += blockDim.x) {
+    const uint32_t t = 4 * (i >> 5) + (i & 3), n = (i & 31) >> 2;  // bytes n & 1 and 2 + (n & 1) of coordinate n / 2
+    const uint32_t x0 = t < terms.n ? reinterpret_cast<const uint32_t*>(&terms.c[t])[n >> 1] : 0;
+    const uint32_t x1 = m31_mul_pow2(x0, 8), x2 = m31_mul_pow2(x0, 16), x3 = m31_mul_pow2(x0, 24);
+    const uint32_t lo = (n & 1) | ((4 + (n & 1)) << 4), hi = lo + 0x22;
+    frag[0][i] = make_uint4(byte_halves(__byte_perm(x0, x1, lo), 0x4140), byte_halves(__byte_perm(x2, x3, lo), 0x4140),
+                            byte_halves(__byte_perm(x0, x1, hi), 0x4140), byte_halves(__byte_perm(x2, x3, hi), 0x4140));
+  }
+  for (uint32_t t = threadIdx.x; t < 4 * steps; t += blockDim.x) ptr[t] = t < terms.n ? terms.col[t] : nullptr;
+  __syncthreads();
+  const uint32_t b_sum = reinterpret_cast<const uint32_t*>(&terms.b_sum)[q];
+  uint32_t* const dst = out.c[q];
+  const uint32_t warps = blockDim.x >> 5;
+#pragma unroll 1
+  for (uint32_t r0 = (blockIdx.x * warps + warp) * kNumRows; r0 < rows; r0 += gridDim.x * warps * kNumRows) {
+    const uint32_t row = r0 + 4 * g;
+    float acc[2][2][2][4];  // [32 rows][2 rows of four][bytes 0, 1 or 2, 3][+ row][+ byte]
+    uint64_t sum[2][4];
+#pragma unroll
+    for (int k = 0; k < 32; k++) (&acc[0][0][0][0])[k] = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) (&sum[0][0])[k] = 0;
+#pragma unroll 1
+    for (uint32_t s0 = 0; s0 < steps; s0 += kNumUnroll) {
+      uint4 v[kNumUnroll][2];
+#pragma unroll
+      for (uint32_t u = 0; u < kNumUnroll; u++) {
+        const uint32_t* p = ptr[4 * (s0 + u) + q];
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          v[u][h] = p != nullptr ? __ldg(reinterpret_cast<const uint4*>(p + row + 32 * h)) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < kNumUnroll; u++) {
+        const uint4 f = frag[s0 + u][lane];
+        const uint32_t b[2][2] = {{f.x, f.y}, {f.z, f.w}};
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const uint32_t w[4] = {v[u][h].x, v[u][h].y, v[u][h].z, v[u][h].w};
+#pragma unroll
+          for (int m = 0; m < 2; m++) {
+            const uint32_t a[4] = {__byte_perm(w[2 * m], 0, 0x4140), __byte_perm(w[2 * m + 1], 0, 0x4140),
+                                   __byte_perm(w[2 * m], 0, 0x4342), __byte_perm(w[2 * m + 1], 0, 0x4342)};
+            mma_f16(acc[h][m][0], a, b[0]);
+            mma_f16(acc[h][m][1], a, b[1]);
+          }
+        }
+      }
+      if (((s0 + kNumUnroll) & 15) != 0 && s0 + kNumUnroll < steps) continue;
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            float& d = acc[h][j >> 1][i >> 1][2 * (j & 1) + (i & 1)];
+            sum[h][j] += (uint64_t)__float2uint_rn(d * 16777216.0f) * (1u << (8 * i));
+            d = 0;
+          }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      uint4* const o = reinterpret_cast<uint4*>(dst + row + 32 * h);
+      uint32_t x[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) x[j] = m31_sub(m31_reduce64(sum[h][j]), b_sum);
+      if (accumulate) {
+        const uint4 old = *o;
+        x[0] = m31_add(x[0], old.x), x[1] = m31_add(x[1], old.y);
+        x[2] = m31_add(x[2], old.z), x[3] = m31_add(x[3], old.w);
+      }
+      *o = make_uint4(x[0], x[1], x[2], x[3]);
+    }
+  }
+}
+
 // ---------------------------------------------------------------- quotients
 
 // Eight rows a thread (see octet_point): the denominators of a sample point are
@@ -1000,7 +1100,17 @@ extern "C" cs_status cs_accumulate_numerators(const uint32_t* const* h_cols, uin
       terms.c[t] = qm31_make(co[8], co[9], co[10], co[11]);
     }
     terms.b_sum = b_sum;
-    numerators_kernel<<<grid_for(rows, 256), 256, 0, to_stream(stream)>>>(terms, rows, o, t0 > 0);
+    // 64-row warps of 16-byte reads; small row counts in blocks of 64 threads, so that more SMs have one
+    bool mma = nt >= kNumMmaMinTerms && rows >= kNumRows;
+    for (int k = 0; k < 4; k++) mma = mma && aligned16(o.c[k]);
+    for (uint32_t t = 0; t < nt; t++) mma = mma && aligned16(terms.col[t]);
+    if (mma) {
+      const uint32_t threads = rows >= 152 * 2 * kNumThreads / 32 * kNumRows ? kNumThreads : 64;
+      const uint32_t blocks = std::min<uint32_t>(rows / (threads / 32 * kNumRows), 152 * 2 * kNumThreads / threads);
+      numerators_mma_kernel<<<std::max(1u, blocks), threads, 0, to_stream(stream)>>>(terms, rows, o, t0 > 0);
+    } else {
+      numerators_kernel<<<grid_for(rows, 256), 256, 0, to_stream(stream)>>>(terms, rows, o, t0 > 0);
+    }
     CS_LAUNCHED("numerators_kernel");
   }
   return CS_OK;

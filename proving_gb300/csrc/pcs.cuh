@@ -7,7 +7,7 @@
 
 namespace cs {
 
-constexpr uint32_t kMaxTerms = 512;   // numerator terms per launch (larger batches are split)
+constexpr uint32_t kMaxTerms = 256;   // numerator terms per launch (larger batches are split)
 constexpr uint32_t kMaxPoints = 16;   // sample points per quotient launch
 
 struct GenPowersTable {
