@@ -190,6 +190,50 @@ __global__ void __launch_bounds__(256) merkle_subtree_kernel(uint32_t* layer, ui
   }
 }
 
+// The three lowest node layers of a tall tree: a thread builds the subtree over eight digests, keeping the
+// nodes it still needs in registers, so that all lanes compress all the time (7/8 of the tree's nodes).
+// Bound: the ALU pipe.
+__global__ void __launch_bounds__(128) merkle_octets_kernel(uint32_t* layer, uint32_t log_in, uint32_t one) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (1u << (log_in - 3))) return;
+  uint32_t first[8], pair[8], h[8];  // a level-1 node, a level-2 node, the last node
+#pragma unroll
+  for (int w = 0; w < 8; w++) first[w] = pair[w] = h[w] = 0;
+#pragma unroll 1
+  for (uint32_t s = 0; s < 7; s++) {  // levels 1 1 2 1 1 2 3
+    const uint32_t level = s == 6 ? 3 : s == 2 || s == 5 ? 2 : 1;
+    const uint32_t node = level == 3 ? i : level == 2 ? 2 * i + (s == 5) : 4 * i + s - (s > 2);
+    uint32_t m[16];
+    if (level == 1) {
+      const uint4* src = reinterpret_cast<const uint4*>(layer + 16 * (size_t)node);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const uint4 w = src[q];
+        m[4 * q] = w.x;
+        m[4 * q + 1] = w.y;
+        m[4 * q + 2] = w.z;
+        m[4 * q + 3] = w.w;
+      }
+    } else {
+#pragma unroll
+      for (int w = 0; w < 8; w++) {
+        m[w] = level == 2 ? first[w] : pair[w];
+        m[8 + w] = h[w];
+      }
+    }
+    b2s_init(h);
+    b2s_compress(h, m, 64, 0, true, one);
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      if (s == 0 || s == 3) first[w] = h[w];
+      if (s == 2) pair[w] = h[w];
+    }
+    uint4* o = reinterpret_cast<uint4*>(layer + 8 * (((size_t)2 << log_in) - ((size_t)2 << (log_in - level)) + node));
+    o[0] = make_uint4(h[0], h[1], h[2], h[3]);
+    o[1] = make_uint4(h[4], h[5], h[6], h[7]);
+  }
+}
+
 // Words from one column to another (columns are word-aligned; unrelated allocations have no pointer
 // difference in C++, so the addresses are subtracted).
 ptrdiff_t word_distance(const uint32_t* a, const uint32_t* b) {
@@ -295,11 +339,14 @@ cs_status merkle_next_layer(const uint32_t* d_prev, uint32_t log_out, uint32_t* 
 
 // Levels built by the next launch over 2^k digests. Measured (all layers of a tree of height h,
 // CUDA events around the call, of which about 10 us are the measurement's own; before: a launch per
-// layer down to 2^10 nodes, then one block): h = 10: 24.8 -> 22.8 us, h = 12: 34.8 -> 25.7,
-// h = 15: 48.3 -> 29.1, h = 17: 60.2 -> 35.9, h = 20: 108 -> 88, h = 22: 241 -> 225. Below 17 eight
+// layer down to 2^10 nodes, then one block): h = 10: 24.8 -> 23.6 us, h = 12: 34.8 -> 25.7,
+// h = 15: 48.3 -> 29.1, h = 17: 60.0 -> 36.9, h = 20: 108 -> 78, h = 22: 241 -> 209. From 19 on a launch
+// of octets first (three levels at full lanes; without it 88 us at h = 20 and 225 at 22; from 18 or 20 on no
+// different); two warps a scheduler or more hide each other's chains there. Else, below 17, eight
 // levels a launch (ten: 33.1 us at h = 15), since the chain counts and eight start with one node a
-// thread; from 17 on ten (eight: 42.3 us at h = 17, 301 at 22), since the blocks fill the chip and
-// the short upper levels are work for few of their warps.
+// thread; at 17 and 18 ten (eight: 42.3 us at h = 17), since the blocks fill the chip and the short
+// upper levels are work for few of their warps.
+constexpr uint32_t kOctetsMinLog = 19;
 uint32_t subtree_levels(uint32_t k) { return k <= 9 ? k : k < 17 ? 8 : kSubtreeMaxLog; }
 
 // Every node layer above the 2^L leaves at d_layers, each right after the one before (leaves
@@ -307,6 +354,13 @@ uint32_t subtree_levels(uint32_t k) { return k <= 9 ? k : k < 17 ? 8 : kSubtreeM
 cs_status merkle_layers(uint32_t* d_layers, uint32_t L, cudaStream_t st) {
   uint32_t* cur = d_layers;
   for (uint32_t k = L; k >= 1;) {
+    if (k >= kOctetsMinLog) {
+      merkle_octets_kernel<<<1u << (k - 3 - 7), 128, 0, st>>>(cur, k, 1u);
+      CS_LAUNCHED("merkle_octets_kernel");
+      cur += 8 * (((size_t)2 << k) - ((size_t)2 << (k - 3)));
+      k -= 3;
+      continue;
+    }
     const uint32_t S = subtree_levels(k);
     const uint32_t threads = std::max(32u, std::min(256u, 1u << (S - 1)));
     const uint32_t blocks = 1u << (k - S);

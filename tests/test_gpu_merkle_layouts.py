@@ -49,7 +49,7 @@ def test_lifted_runs(layout, logs, height):
     assert B.merkle_commit(cols, height).root() == O.merkle_commit(vals, height)
 
 
-@pytest.mark.parametrize("height", [1, 2, 5, 8, 9, 10, 11, 16, 17, 18, 19])
+@pytest.mark.parametrize("height", [1, 2, 5, 8, 9, 10, 11, 16, 17, 18, 19, 20, 21, 22])
 def test_every_layer(height):
     from proving_gb300.backend import CudaBackend as B
     vals = m31_columns(height, 2, height)
