@@ -32,7 +32,7 @@ def _check(vals, weights, offset=0):
         assert np.array_equal(g, O.barycentric_eval(v, weights))
 
 
-@pytest.mark.parametrize("log_n,n_cols", [(11, 3), (12, 1), (12, 16), (12, 17), (13, 15), (14, 33), (16, 257), (17, 40),
+@pytest.mark.parametrize("log_n,n_cols", [(11, 3), (12, 1), (12, 7), (12, 8), (18, 9), (12, 16), (12, 17), (13, 15), (14, 33), (16, 257), (17, 40),
                                           (20, 5)])
 def test_evaluation(log_n, n_cols):
     x, y = pr.random_point(tuple(int(v) for v in seeded_qm31(log_n)))
