@@ -56,7 +56,7 @@ def workload_name():
 
 # DRAM bytes (read + write) measured with ncu on the 256 x 2^20 workload
 # (profiles/launch_list_commit_stage_256x2^20.md): one merkle_leaves_kernel launch, and the two
-# fft_tile_kernel launches of one evaluate
+# FFT pass launches of one evaluate
 LEAVES_TRAFFIC_BYTES = 4425.2e6
 EVALUATE_TRAFFIC_BYTES = 13935.0e6
 
@@ -907,7 +907,7 @@ def run_gpu(args):
         return
     hbm, peak_kind = peaks()
     default_shape = (N_COLS, LOG_ROWS, LOG_EXT) == (256, 20, 22)
-    # dominant kernel: the evaluate FFT (fft_tile_kernel, two tile passes per step); algorithmic
+    # dominant kernels: the evaluate FFT (a strided and a contiguous pass per step); algorithmic
     # bytes per column are 4 n_in + 4 n_out (coefficients read once, the blown-up evaluation written)
     eval_ms = stage_ms["evaluate"]
     eval_bytes = N_COLS * 4 * ((1 << LOG_ROWS) + (1 << LOG_EXT))
@@ -935,13 +935,13 @@ def run_gpu(args):
                        "e2e_p50": ff(float(np.percentile(e_lat, 50))), "e2e_p99": ff(float(np.percentile(e_lat, 99)))},
         "stages_ms": {k: ff(v) for k, v in stage_ms.items()},
         "e2e": {"value": ff(e2e_value), "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-        "roofline": {"bound": "hbm", "kernel": "fft_tile_kernel (evaluate: 2 tile passes per step)",
+        "roofline": {"bound": "hbm", "kernel": "fft_strided_kernel + fft_contig_kernel (evaluate: 2 passes per step)",
                      "achieved": ff(achieved), "peak": hbm, "unit": "GB/s", "frac": ff(achieved / hbm),
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json)", "traffic": eval_traffic,
                      "algorithmic_bytes_per_evaluate": eval_bytes, "launches_per_evaluate": 2,
                      "note": "achieved and traffic are per evaluate (both passes); the passes are bound by "
-                             "integer issue (about 11.4 thread instructions per butterfly, most of them the "
-                             "M31 multiply-reduce and the two reduced additions), and traffic counts the "
+                             "integer issue (a butterfly is 7 instructions and 10.85 cycles of a warp in registers: "
+                             "the M31 multiply-reduce and the two reduced additions), and traffic counts the "
                              "intermediate of the two-pass FFT written once and read once"},
         "leaves_roofline": {"bound": "hbm", "kernel": "merkle_leaves_kernel", "achieved": ff(leaf_gbs), "peak": hbm,
                             "unit": "GB/s", "frac": ff(leaf_gbs / hbm), "traffic": traffic,

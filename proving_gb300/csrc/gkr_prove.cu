@@ -16,9 +16,10 @@
 //
 // Bound: latency (7.3 us a round in the single-block kernel, 13 in a launch of its own: 4.6 for the
 // terms, 1.5 for the blocks' sums, 4.7 to end the round, 0.7 to the next launch). A QM31 product is
-// 155-220 cycles for a lone warp and a compression about 1,900, so the block spreads a round's products over its threads in as few levels as they need: one product per
-// element to fix, two per part of a term, one per (coefficient, sum), and what only the next round
-// needs (claims, corrections, coefficient tables) runs in other warps beside the next fix.
+// 155-220 cycles for a lone warp and a compression about 1,900, so the block spreads a round's products over
+// its threads in as few levels as they need: one product per element to fix, two per part of a term, one per
+// (coefficient, sum), and what only the next round needs (claims, corrections, coefficient tables) runs in
+// other warps beside the next fix.
 #include <algorithm>
 #include <cstddef>
 #include <cstring>

@@ -486,7 +486,11 @@ struct LookupCompParams {
 
 // Quotients of single-column LogUp components of one size: per evaluation row, the sum over the
 // components of rc (cur - prev + shift) (v - z) + 1, over V_trace, added to the accumulator once.
-// Components go in pairs whose 18 loads are issued before either is evaluated.
+// Components go in pairs whose 18 loads are issued before either is evaluated. The 256-row tiles are taken
+// in bit-reversed order: a tile's previous rows lie in the tiles whose reversed numbers are next to its own,
+// which are then in flight at the same time, and their second read hits L2. Bound: the ALU pipe and HBM
+// alike (20 M31 products and 36 bytes, 20 of them from HBM, a component row). 120 components of 2^10 to 2^22
+// rows: 2.56 -> 2.35 ms.
 struct LookupRow {
   uint32_t v, cur[4], prev[4];
 };
@@ -512,8 +516,10 @@ __device__ __forceinline__ qm31 lookup_term(const LookupCompParams& p, uint32_t 
 
 __global__ void lookup_composition_kernel(const __grid_constant__ LookupCompParams p, uint32_t* a0, uint32_t* a1,
                                           uint32_t* a2, uint32_t* a3) {
-  const uint32_t n = 1u << p.eval_log;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+  const uint32_t tile_log = p.eval_log > 8 ? p.eval_log - 8 : 0;
+  if (threadIdx.x >> min(p.eval_log, 8u)) return;
+  for (uint32_t tile = blockIdx.x; tile >> tile_log == 0; tile += gridDim.x) {
+    const uint32_t r = rev_bits(tile, tile_log) << 8 | threadIdx.x;
     const uint32_t pr = prev_row(r, p.trace_log, p.eval_log);
     qm31 acc = p.rc_sum;
     uint32_t k = 0;
