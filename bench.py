@@ -1244,7 +1244,7 @@ def gkr_leg(torch, log_logup: int = 22, log_gp: int = 20, n_proofs: int = 3, ker
             "native_equals_driver": bool(same),
             "kernels": kernels,
             "note": "prove_p50_ms: the protocol in Python over the device ops (proving_gb300.gkr.prove_batch); "
-                    "native_prove_p50_ms: the protocol in C++ (cs_gkr_prove_batch), one read-back per round"}
+                    "native_prove_p50_ms: the protocol on the device (cs_gkr_prove_batch), one read-back per proof"}
 
 
 def run_case(args):

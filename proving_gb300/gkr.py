@@ -553,7 +553,7 @@ class DeviceGkrOps:
 
 def prove_batch_native(channel, input_layers) -> tuple[GkrBatchProof, GkrArtifact]:
     """prove_batch with the protocol in native code (cs_gkr_prove_batch): the same proof and
-    artifact as prove_batch over DeviceGkrOps, with one host synchronisation per sum-check round and
+    artifact as prove_batch over DeviceGkrOps, with one host synchronisation per proof and
     no interpreter between the launches. Inputs are device MLEs (DeviceGkrOps' layout); the
     channel (proving_gb300.prover.Blake2sChannel) is advanced as prove_batch advances it."""
     import struct
