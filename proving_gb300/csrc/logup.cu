@@ -142,20 +142,17 @@ __device__ __forceinline__ void warp_scan4(uint32_t x[4]) {
   }
 }
 
-// The warp's sum of r[0..3] (each below P): coordinate lane >> 3 in lanes 0, 8, 16, 24. The first two
-// steps halve the coordinates a lane keeps: 6 shuffles instead of 20.
-__device__ __forceinline__ uint32_t warp_sum4(const uint32_t r[4], uint32_t lane) {
-  const bool hi = (lane >> 4) & 1;  // keeps coordinates 2, 3
+// The sum of r[0..3] (each below P) over eight neighbouring lanes: coordinate (lane >> 1) & 3 in all of them.
+// The first two steps halve the coordinates a lane keeps: 4 shuffles instead of 12.
+__device__ __forceinline__ uint32_t sum4_of_eight(const uint32_t r[4], uint32_t lane) {
+  const bool hi = (lane >> 2) & 1;  // keeps coordinates 2, 3
   uint32_t k0 = hi ? r[2] : r[0], k1 = hi ? r[3] : r[1];
-  const uint32_t s0 = hi ? r[0] : r[2], s1 = hi ? r[1] : r[3];
-  k0 = m31_add(k0, __shfl_xor_sync(0xffffffffu, s0, 16));
-  k1 = m31_add(k1, __shfl_xor_sync(0xffffffffu, s1, 16));
-  const bool odd = (lane >> 3) & 1;  // keeps the second of its pair
+  k0 = m31_add(k0, __shfl_xor_sync(0xffffffffu, hi ? r[0] : r[2], 4));
+  k1 = m31_add(k1, __shfl_xor_sync(0xffffffffu, hi ? r[1] : r[3], 4));
+  const bool odd = (lane >> 1) & 1;  // keeps the second of its pair
   uint32_t v = odd ? k1 : k0;
-  v = m31_add(v, __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 8));
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) v = m31_add(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  v = m31_add(v, __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 2));
+  return m31_add(v, __shfl_xor_sync(0xffffffffu, v, 1));
 }
 
 // A column of at most 2^9 rows, all in one block (at least 2^9 threads).
@@ -219,13 +216,13 @@ __device__ __forceinline__ void fraction_quad(const qm31& z, const uint32_t (&v)
   }
 }
 
-// Launch 1 (256 threads): per tile m of a column of 2^10 or more rows,
-// thread (w, t) (w < 8) takes the storage positions (rev5(lo) << (l - 5)) | (rev(m) << 5) | t for
-// lo = w + 8 q, q < 4, i.e. natural (h = rev5(t), m, lo); its four fractions share one M31 inversion and
-// its four loads are in flight together. Bound: the inversion's chain and HBM (4 bytes read, 16 written a
-// row). One position a thread, 1,024 threads and an inversion each took 1.75 ms over the 120 columns (2^10
-// to 2^22 rows) of a mixed proof; this takes 1.13 ms. Columns of 2^9 rows or fewer have a kernel of their
-// own so that its registers and shared memory are not this one's.
+// Launch 1 (256 threads): per tile m of a column of 2^10 or more rows, thread (w, t) (w < 8) takes the storage
+// positions (rev5(lo) << (l - 5)) | (rev(m) << 5) | t for lo = w + 8 q, q < 4, i.e. natural
+// (h = rev5(t), m, lo); its four fractions share one M31 inversion and its four loads are in flight
+// together. Bound: issue (ALU pipe 61%, 2.6 of 4 slots; DRAM 19%): about 40 products a row. Over the 120 columns
+// (2^10 to 2^22 rows) of a mixed proof: two rows a thread 1.75 ms, four 1.13, with a run's total summed by eight
+// lanes of four values (4 shuffles for four runs instead of 24) 1.05. Columns of 2^9 rows or fewer have a kernel
+// of their own so that its registers and shared memory are not this one's.
 __global__ void __launch_bounds__(kTileThreads) runs_kernel(const SumBatch b) {
   __shared__ uint32_t tile[4][32][33];
   const uint32_t col = block_column(b.tile0, b.n_cols, blockIdx.x);
@@ -257,16 +254,14 @@ __global__ void __launch_bounds__(kTileThreads) runs_kernel(const SumBatch b) {
     tile[3][lo][h] = g[q].b.b;
   }
   __syncthreads();
-  // warp w sums natural runs (h' = w + 8 q, m): lanes are lo
+  // eight lanes sum the natural run (hh, m), four consecutive lo each (reads free of bank conflicts)
+  const uint32_t hh = 4 * w + (t >> 3), lo = 4 * (t & 7);
+  uint32_t x[4];
 #pragma unroll
-  for (int q = 0; q < kQuad; q++) {
-    const uint32_t hh = w + 8 * q;
-    uint32_t x[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) x[k] = tile[k][t][hh];
-    const uint32_t v = warp_sum4(x, t);  // coordinate t / 8, in lanes 0, 8, 16, 24
-    if ((t & 7) == 0) b.runs[4 * (b.run0[col] + ((hh << mb) | m)) + (t >> 3)] = v;
-  }
+  for (int k = 0; k < 4; k++)
+    x[k] = m31_add(m31_add(tile[k][lo][hh], tile[k][lo + 1][hh]), m31_add(tile[k][lo + 2][hh], tile[k][lo + 3][hh]));
+  const uint32_t v = sum4_of_eight(x, t);
+  if ((t & 1) == 0) b.runs[4 * (b.run0[col] + ((hh << mb) | m)) + ((t >> 1) & 3)] = v;
 }
 
 // Columns of at most 2^9 rows: one block each.
@@ -331,11 +326,11 @@ __global__ void __launch_bounds__(kThreads) run_offsets_kernel(const SumBatch b)
   }
 }
 
-// Launch 3 (256 threads): per mirror pair of tiles (m, m' = ~m) of a column of 2^10 or more rows; a thread
-// has four elements of each tile, whose loads are in flight together. Bound: HBM (16 bytes read, 16 written
-// a row; the second read of a fraction hits L1 or L2) and the scans' shuffles. With 1,024 threads of one
-// element the three waves of a block left the memory idle in between: 2.17 ms for the same 120 columns,
-// 1.49 ms here.
+// Launch 3 (256 threads): per mirror pair of tiles (m, m' = ~m) of a column of 2^10 or more rows; a thread has
+// four elements of each tile, whose loads are in flight together, and eight lanes scan a run, four values
+// each (16 shuffles for four runs; 80 with a lane a value). Bound: latency between its three waits and the
+// scattered halves of a fraction's second read (DRAM 27%, ALU pipe 44%). For the same 120 columns: 1,024
+// threads of one element 2.17 ms, four elements 1.49, the runs by eight lanes 1.30.
 __global__ void __launch_bounds__(kTileThreads) outputs_kernel(const SumBatch b) {
   __shared__ uint32_t tiles[2][4][32][33];
   const uint32_t col = block_column(b.pair0, b.n_cols, blockIdx.x);
@@ -366,19 +361,27 @@ __global__ void __launch_bounds__(kTileThreads) outputs_kernel(const SumBatch b)
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     if ((uint32_t)q >= n_tiles) break;
+    // prefixes of the natural run (hh, ms[q]): eight lanes, four consecutive lo each
+    const uint32_t hh = 4 * w + (t >> 3), lane = t & 7;
+    const uint4 run = r[(hh << mb) | ms[q]], seg = hoff[hh];
+    const uint32_t off[4] = {m31_add(run.x, seg.x), m31_add(run.y, seg.y), m31_add(run.z, seg.z), m31_add(run.w, seg.w)};
 #pragma unroll
-    for (int j = 0; j < kQuad; j++) {
-      // natural run (hh, ms[q]); lanes are lo
-      const uint32_t hh = w + 8 * j;
-      uint32_t x[4];
+    for (int k = 0; k < 4; k++) {
+      uint32_t x[kQuad];
 #pragma unroll
-      for (int k = 0; k < 4; k++) x[k] = tiles[q][k][t][hh];
-      const uint4 run = r[(hh << mb) | ms[q]], seg = hoff[hh];
-      warp_scan4(x);
-      tiles[q][0][t][hh] = m31_add(x[0], m31_add(run.x, seg.x));
-      tiles[q][1][t][hh] = m31_add(x[1], m31_add(run.y, seg.y));
-      tiles[q][2][t][hh] = m31_add(x[2], m31_add(run.z, seg.z));
-      tiles[q][3][t][hh] = m31_add(x[3], m31_add(run.w, seg.w));
+      for (int i = 0; i < kQuad; i++) x[i] = tiles[q][k][4 * lane + i][hh];
+#pragma unroll
+      for (int i = 1; i < kQuad; i++) x[i] = m31_add(x[i], x[i - 1]);
+      uint32_t sum = x[kQuad - 1];
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, sum, o, 8);
+        if (lane >= (uint32_t)o) sum = m31_add(sum, y);
+      }
+      const uint32_t before = __shfl_up_sync(0xffffffffu, sum, 1, 8);
+      const uint32_t base = lane == 0 ? off[k] : m31_add(off[k], before);
+#pragma unroll
+      for (int i = 0; i < kQuad; i++) tiles[q][k][4 * lane + i][hh] = m31_add(x[i], base);
     }
   }
   __syncthreads();
