@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fft_layout.cuh"
 #include "field.cuh"
 
 namespace cs {
@@ -606,22 +607,6 @@ __global__ void __launch_bounds__(32 * kContigWarps, direct_min_blocks<T - T / 2
   }
 }
 
-// A strided tile holds [m][e] with 8 pad words per stage row (2^TA values of m), so that a warp's
-// four rows fall on distinct banks.
-template <int TA, int EB>
-__device__ __forceinline__ constexpr uint32_t strided_pad(uint32_t L) {
-  return L + ((L >> (TA + EB)) << EB);
-}
-template <int T, int EB>
-constexpr uint32_t strided_tile_words() {
-  return (1u << (EB + T)) + (1u << (EB + T - T / 2));
-}
-template <int T, int EB>
-constexpr uint32_t strided_smem_words() {
-  constexpr int TA = T / 2, TB = T - TA;
-  return strided_tile_words<T, EB>() + (1u << TB) + (((1u << EB) << TA) / 32) * ((32u >> EB) << TB);
-}
-
 // Layers [lo, lo + T), lo >= 3: a block owns the 2^T values of 8 neighbouring groups (32-byte runs
 // in memory), one (group, stage row) a thread.
 template <bool INV, int T, int EB>
@@ -632,9 +617,10 @@ __global__ void __launch_bounds__((1 << EB) << (T / 2), direct_min_blocks<T - T 
   const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31;
   constexpr int RW = 32 >> EB;  // rows a warp
   const uint32_t e = t & ((1u << EB) - 1), ml = t >> EB;
-  // every warp writes the same words to the high stage's table, which depends on the block alone
-  uint32_t* tabB = smem + strided_tile_words<T, EB>();
-  uint32_t* tabA = tabB + (1 << TB) + warp * (RW << TB);
+  // each warp has a copy of the high stage's table, which depends on the block alone: no barrier
+  // between the fill and the first stage
+  uint32_t* tabB = smem + strided_high_table<T, EB>(warp);
+  uint32_t* tabA = smem + strided_low_table<T, EB>(warp);
   // replicated reads (evaluate's first pass): the replicas of a tile are neighbouring blocks and
   // share its reads; otherwise neighbouring runs of the same lines are
   const uint32_t outer_bits = p.log_n - p.hi, run_bits = p.lo - EB;
