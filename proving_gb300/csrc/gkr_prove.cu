@@ -54,7 +54,7 @@ struct LayerCols {
   const uint32_t *num[4], *den[4];
   uint32_t *fnum[4], *fden[4];
   uint32_t kind;
-  uint32_t n_vars;
+  uint32_t n_vars;  // variables of the layer; 0 before the instance joins
 };
 
 // The round polynomial is linear in the sums f0, f2 at t = 0, 2 and the claim:
@@ -626,12 +626,16 @@ __global__ void __launch_bounds__(kRoundThreads) gkr_round_kernel(const GkrProgr
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ bool last;
   __shared__ qm31 part[4][kRoundThreads / 32];
-  const uint32_t i = blockIdx.y, delta = g.inst[i].delta, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t i = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // how late the instance joins, from the table that no launch of the chain writes (InstState, which the
+  // launch before this one writes back, may only be read after the wait)
+  const LayerCols& L = g.cols[(size_t)layer * g.n_inst + i];
+  const uint32_t delta = layer + 1 - L.n_vars;
   hash_setup(*reinterpret_cast<Hash*>(smem + sizeof(GkrState)));
   chain_wait();
   const Block B = prefetch_block(g, smem, layer, round);
   if (delta <= round) {
-    const Sums s = round_terms(g.cols[(size_t)layer * g.n_inst + i], round - delta, 1u << (layer - round - 1),
+    const Sums s = round_terms(L, round - delta, 1u << (layer - round - 1),
                                blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, g.eq, 1u << (layer - 1),
                                g.state->x);
     const qm31 w[4] = {warp_sum(s.a0), warp_sum(s.c0), warp_sum(s.a2), warp_sum(s.c2)};
