@@ -1061,7 +1061,8 @@ cs_status gkr_prove_on_device(const std::vector<GkrInput>& inputs, uint32_t chan
   g.eq = eq;
 
   const size_t round_bytes = block_bytes(n_inst), tail_bytes = tail_smem(n_inst);
-  cs_status attr = allow_smem(gkr_tail_kernel, tail_smem(kSharedCols), 0);
+  // the tail's largest: tail columns of kSharedCols instances, or the state of kSharedInst
+  cs_status attr = allow_smem(gkr_tail_kernel, std::max(tail_smem(kSharedCols), tail_smem(kSharedInst)), 0);
   if (attr == CS_OK) attr = allow_smem(gkr_round_kernel, block_bytes(kSharedInst), 1);
   if (attr != CS_OK) return attr;
   attr = allow_smem(gkr_start_kernel, block_bytes(kSharedInst), 2);
