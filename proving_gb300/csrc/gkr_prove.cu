@@ -916,11 +916,13 @@ struct Buffers {
     for (void* p : ptrs) cudaFreeAsync(p, st);
   }
   template <typename T>
-  T* get(size_t n) {
+  cs_status get(T*& out, size_t n) {
     void* p = nullptr;
-    if (stream_alloc(&p, std::max<size_t>(16, n * sizeof(T)), st) != cudaSuccess) return nullptr;
+    const cudaError_t e = stream_alloc(&p, std::max<size_t>(16, n * sizeof(T)), st);
+    if (e != cudaSuccess) return from_cuda(e, "gkr_prove_batch: allocation");
     ptrs.push_back(p);
-    return static_cast<T*>(p);
+    out = static_cast<T*>(p);
+    return CS_OK;
   }
 };
 
@@ -964,12 +966,9 @@ cs_status gkr_prove_on_device(const std::vector<GkrInput>& inputs, uint32_t chan
     // the input's first fix goes to scratch of half its size, behind the stack
     const size_t half = (size_t)4 << (in.n_vars - 1);
     const bool fix_num = in.kind == CS_GKR_LOGUP_GENERIC || in.kind == CS_GKR_LOGUP_MULTIPLICITIES;
-    s.den = mem.get<uint32_t>(words + half);
-    if (s.den == nullptr) return CS_ERR_OOM;
-    if (!product) {
-      s.num = mem.get<uint32_t>(words + (fix_num ? half : 0));
-      if (s.num == nullptr) return CS_ERR_OOM;
-    }
+    cs_status a = mem.get(s.den, words + half);
+    if (a == CS_OK && !product) a = mem.get(s.num, words + (fix_num ? half : 0));
+    if (a != CS_OK) return a;
     const uint32_t* num[4] = {in.num[0], in.num[1], in.num[2], in.num[3]};
     const uint32_t* den[4] = {in.den[0], in.den[1], in.den[2], in.den[3]};
     uint32_t kind = in.kind;
@@ -1039,10 +1038,11 @@ cs_status gkr_prove_on_device(const std::vector<GkrInput>& inputs, uint32_t chan
   const size_t at_outputs = (at_masks + masks_bytes + 15) & ~(size_t)15, outputs_bytes = 4 * 8 * (size_t)n_inst;
   const size_t at_partial = (at_outputs + outputs_bytes + 15) & ~(size_t)15;
   const size_t total = at_partial + 4 * 16 * (size_t)n_inst * max_blocks;
-  unsigned char* dev = mem.get<unsigned char>(total);
-  if (dev == nullptr) return CS_ERR_OOM;
-  uint32_t* eq = mem.get<uint32_t>((size_t)4 << max_terms_log);
-  if (eq == nullptr) return CS_ERR_OOM;
+  unsigned char* dev = nullptr;
+  uint32_t* eq = nullptr;
+  cs_status a = mem.get(dev, total);
+  if (a == CS_OK) a = mem.get(eq, (size_t)4 << max_terms_log);
+  if (a != CS_OK) return a;
   CS_CUDA(cudaMemcpyAsync(dev, up.bytes.data(), up.bytes.size(), cudaMemcpyHostToDevice, st));
 
   GkrProgram g;

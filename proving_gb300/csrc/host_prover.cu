@@ -204,8 +204,9 @@ struct Arena {
   explicit Arena(cudaStream_t s) : st(s) {}
   uint32_t* alloc(size_t words) {
     void* p = nullptr;
-    if (stream_alloc(&p, std::max<size_t>(4, 4 * words), st) != cudaSuccess) {
-      status = CS_ERR_OOM;
+    const cudaError_t e = stream_alloc(&p, std::max<size_t>(4, 4 * words), st);
+    if (e != cudaSuccess) {
+      status = from_cuda(e, "prover: allocation");
       return nullptr;
     }
     ptrs.push_back(p);

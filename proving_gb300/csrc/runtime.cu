@@ -47,6 +47,7 @@ void set_error(const char* fmt, ...) {
 }
 
 cs_status from_cuda(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here: the next launch's check must not find it again
   set_error("%s: %s (%s)", what, cudaGetErrorString(e), cudaGetErrorName(e));
   if (e == cudaErrorMemoryAllocation) return CS_ERR_OOM;
   if (e == cudaErrorInvalidValue) return CS_ERR_INVALID_ARG;
