@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(32 * kContigWarps, direct_min_blocks<T - T / 2
     if (p.scale) {
       const uint32_t k = __ffs(p.scale) - 1;
 #pragma unroll
-      for (int j = 0; j < V; j++) v[j] = m31_mul_pow2(v[j], k);
+      for (int j = 0; j < V; j++) v[j] = m31_reduce_once(m31_mul_pow2(v[j], k));  // P, a zero of the input, to 0
     }
 #pragma unroll
     for (int j = 0; j < V; j++) q[j << TA] = v[j];
@@ -689,7 +689,7 @@ __global__ void __launch_bounds__((1 << EB) << (T / 2), direct_min_blocks<T - T 
     if (p.scale) {
       const uint32_t k = __ffs(p.scale) - 1;
 #pragma unroll
-      for (int j = 0; j < V; j++) v[j] = m31_mul_pow2(v[j], k);
+      for (int j = 0; j < V; j++) v[j] = m31_reduce_once(m31_mul_pow2(v[j], k));  // P, a zero of the input, to 0
     }
     uint32_t* q = dst + ((size_t)ml << p.lo);
 #pragma unroll

@@ -24,7 +24,8 @@ __host__ __device__ __forceinline__ uint32_t m31_mul(uint32_t a, uint32_t b) {
   const uint64_t p = (uint64_t)a * (uint64_t)(b + b);
   return m31_reduce_once(((uint32_t)p >> 1) + (uint32_t)(p >> 32));
 }
-// x 2^k mod P for a canonic x and 0 < k < 31: a rotation of its 31 bits.
+// x 2^k mod P for a canonic x and 0 < k < 31: a rotation of its 31 bits. The word P, which counts as
+// zero, stays P, where m31_mul gives 0.
 __host__ __device__ __forceinline__ uint32_t m31_mul_pow2(uint32_t x, uint32_t k) {
   return ((x << k) & P) | (x >> (31 - k));
 }
