@@ -31,10 +31,44 @@ __device__ __forceinline__ uint32_t fold64(uint64_t v) {
   return m31_reduce_once((uint32_t)((t & P) + (t >> 31)));
 }
 
+// A row a thread, the constraints one after another. Lazy sums: each weight x constraint product is
+// below 2^62 and is added unreduced (one 64-bit multiply-add per coordinate); folding every four
+// constraints keeps the sums below 2^64 (a fold leaves less than 2^34). Each column is squared once, for
+// the constraint that reads it as b and the next one that reads it as a.
+__global__ void __launch_bounds__(256) wide_fib_rows_kernel(const __grid_constant__ WideFibParams p, uint32_t* a0,
+                                                             uint32_t* a1, uint32_t* a2, uint32_t* a3) {
+  const uint32_t n = 1u << p.eval_log;
+  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    uint64_t acc[4] = {0, 0, 0, 0};
+    uint32_t sa = m31_sqr(__ldg(p.cols[0] + r)), sb = m31_sqr(__ldg(p.cols[1] + r));
+    for (uint32_t k = 0; k + 2 < p.n_cols; k++) {
+      const uint32_t c = __ldg(p.cols[k + 2] + r);
+      const uint32_t cons = m31_sub(c, m31_add(sa, sb));
+      const qm31 w = p.rc[k];
+      acc[0] += (uint64_t)w.a.a * cons;
+      acc[1] += (uint64_t)w.a.b * cons;
+      acc[2] += (uint64_t)w.b.a * cons;
+      acc[3] += (uint64_t)w.b.b * cons;
+      if ((k & 3) == 3) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[j] = (acc[j] & P) + (acc[j] >> 31);
+      }
+      sa = sb;
+      sb = m31_sqr(c);
+    }
+    const uint32_t d = p.den[r >> p.trace_log];
+    a0[r] = m31_add(a0[r], m31_mul(fold64(acc[0]), d));
+    a1[r] = m31_add(a1[r], m31_mul(fold64(acc[1]), d));
+    a2[r] = m31_add(a2[r], m31_mul(fold64(acc[2]), d));
+    a3[r] = m31_add(a3[r], m31_mul(fold64(acc[3]), d));
+  }
+}
+
 // A warp takes 32 rows and one of `split` runs of the constraints; the runs of a row group are warps of
 // one block and meet in shared memory. Columns are loaded eight ahead of the constraint that reads
-// them: one at a time, the loop waited for every load (36 us for the 98 constraints of 2^15 rows).
+// them: one at a time, the loop waited for every load (98 constraints of 2^15 rows: 15.2 us, 9.0 here).
 constexpr int kFibWarps = 8, kFibAhead = 8;
+constexpr uint32_t kFibSplitThreads = 1u << 16;
 
 __global__ void __launch_bounds__(32 * kFibWarps) wide_fib_composition_kernel(const __grid_constant__ WideFibParams p,
                                                                               uint32_t split, uint32_t* a0,
@@ -48,11 +82,7 @@ __global__ void __launch_bounds__(32 * kFibWarps) wide_fib_composition_kernel(co
   uint32_t* const out[4] = {a0, a1, a2, a3};
   for (uint32_t base = blockIdx.x * groups * 32; base < n; base += gridDim.x * groups * 32) {
     const uint32_t r = base + group * 32 + lane;
-    // Lazy sums: each weight x constraint product is below 2^62 and is added unreduced (one
-    // 64-bit multiply-add per coordinate); folding every four constraints keeps the sums below
-    // 2^64 (a fold leaves less than 2^34). Each column is squared once, for the constraint that
-    // reads it as b and the next one that reads it as a.
-    uint64_t acc[4] = {0, 0, 0, 0};
+    uint64_t acc[4] = {0, 0, 0, 0};  // lazy sums, as in wide_fib_rows_kernel
     if (r < n && k0 < k1) {
       uint32_t sa = m31_sqr(__ldg(p.cols[k0] + r)), sb = m31_sqr(__ldg(p.cols[k0 + 1] + r));
       uint32_t next[kFibAhead];
@@ -175,9 +205,23 @@ extern "C" cs_status cs_wide_fib_composition(const uint32_t* const* h_cols, uint
   }
   for (int c = 0; c < 4; c++) CS_CHECK_ARG(h_accum[c] != nullptr, "wide_fib_composition: null accumulator");
   const uint32_t n = 1u << eval_log;
-  // runs of eight constraints and more, as many as it takes for the chip's 2048 threads an SM
+  // Device us, columns in L2 (rows kernel / 1, 2, 4, 8 runs):
+  //   100 columns of 2^13 14.6 / 11.2, 7.4, 5.5, 4.8; of 2^14 15.2 / 11.4, 7.6, 6.3, 6.7; of 2^15 15.2 / 11.5,
+  //   9.0, 9.6, 10.1; of 2^16 16.1 / 14.4, 15.0, 15.1, 16.4; of 2^18 51.9 / 43.8, 45.9, 56.6, 68.2
+  // so as many runs (of eight constraints or more) as make 2^16 threads: more of them walk different
+  // columns' pointers and weights, which then miss the constant cache (256 columns of 2^16: one run 31.8,
+  // eight 49.7). Few constraints are not worth the runs' look-ahead:
+  //   3 columns of 2^10 2.4 / 2.8, of 2^20 8.4 / 17.6; 10 of 2^12 3.5 / 3.3, of 2^20 19.5 / 22.7;
+  //   18 of 2^18 9.8 / 10.7; 34 of 2^18 16.0 / 16.4, of 2^19 31.3 / 29.1
+  const uint32_t n_con = n_cols - 2;
+  if (n_con < 8 || (n_con <= 16 && n >= kFibSplitThreads)) {
+    wide_fib_rows_kernel<<<std::max(1u, std::min((n + 255) / 256, 152u * 8)), 256, 0, to_stream(stream)>>>(
+        p, h_accum[0], h_accum[1], h_accum[2], h_accum[3]);
+    CS_LAUNCHED("wide_fib_rows_kernel");
+    return CS_OK;
+  }
   uint32_t split = 1;
-  while (split < (uint32_t)kFibWarps && (uint64_t)n * split < 152ull * 2048 && (n_cols - 2) / (2 * split) >= 8) split *= 2;
+  while (split < (uint32_t)kFibWarps && (uint64_t)n * split < kFibSplitThreads && n_con / (2 * split) >= 8) split *= 2;
   const uint32_t rows = 32 * (kFibWarps / split);
   const uint32_t blocks = std::max(1u, std::min((n + rows - 1) / rows, 152u * 8));
   wide_fib_composition_kernel<<<blocks, 32 * kFibWarps, 0, to_stream(stream)>>>(p, split, h_accum[0], h_accum[1],
