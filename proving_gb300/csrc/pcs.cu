@@ -548,7 +548,8 @@ __global__ void eval_at_point_kernel(const BaryColumns cols, const FoldFactors f
 // row r: sum_t c_t * col_t[r] - sum_t b_t (the batch's partial numerator). Terms go in groups of 8:
 // the 8 column values are loaded first, then their unreduced 64-bit products are added, folded below
 // 2^34 after every 4 (4 products below P^2 < 2^62 on top of a folded value stay below 2^64).
-__global__ void numerators_kernel(const NumeratorTerms terms, uint32_t rows, SoA out, bool accumulate) {
+template <uint32_t N>
+__global__ void numerators_kernel(const NumeratorTerms<N> terms, uint32_t rows, SoA out, bool accumulate) {
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
     uint64_t a[4] = {0, 0, 0, 0};
     uint32_t t = 0;
@@ -601,11 +602,11 @@ constexpr uint32_t kNumUnroll = 4;
 // here against 30.7 by multiply-adds, 26 of 2^22 101 against 115.
 constexpr uint32_t kNumMmaMinTerms = 25;
 
-__global__ void __launch_bounds__(kNumThreads, 2) numerators_mma_kernel(const __grid_constant__ NumeratorTerms terms,
-                                                                        uint32_t rows, const __grid_constant__ SoA out,
-                                                                        bool accumulate) {
-  __shared__ uint4 frag[kMaxTerms / 4][32];
-  __shared__ const uint32_t* ptr[kMaxTerms];
+__global__ void __launch_bounds__(kNumThreads, 2) numerators_mma_kernel(
+    const __grid_constant__ NumeratorTerms<kMmaTerms> terms, uint32_t rows, const __grid_constant__ SoA out,
+    bool accumulate) {
+  __shared__ uint4 frag[kMmaTerms / 4][32];
+  __shared__ const uint32_t* ptr[kMmaTerms];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const uint32_t steps = (terms.n + 4 * kNumUnroll - 1) / (4 * kNumUnroll) * kNumUnroll;
   for (uint32_t i = threadIdx.x; i < steps * 32; i += blockDim.x) {
@@ -1068,6 +1069,21 @@ extern "C" cs_status cs_eval_at_point(const uint32_t* const* h_coeffs, uint32_t 
   return CS_OK;
 }
 
+// n terms of 12 coefficient words (a, b, c) each as a launch's parameters.
+template <uint32_t N>
+static const NumeratorTerms<N>& numerator_terms(const uint32_t* const* cols, const uint32_t* coeffs, uint32_t n) {
+  static thread_local NumeratorTerms<N> terms;
+  terms.n = n;
+  terms.b_sum = qm31_make(0, 0, 0, 0);
+  for (uint32_t t = 0; t < n; t++) {
+    const uint32_t* co = coeffs + 12 * t;
+    terms.col[t] = cols[t];
+    terms.b_sum = qm31_add(terms.b_sum, qm31_make(co[4], co[5], co[6], co[7]));
+    terms.c[t] = qm31_make(co[8], co[9], co[10], co[11]);
+  }
+  return terms;
+}
+
 extern "C" cs_status cs_accumulate_numerators(const uint32_t* const* h_cols, uint32_t n_terms, uint32_t log_size,
                                               uint32_t log_blowup, const uint32_t* h_coeffs,
                                               uint32_t* const h_out[4], uint32_t first_linear_out[4],
@@ -1091,28 +1107,28 @@ extern "C" cs_status cs_accumulate_numerators(const uint32_t* const* h_cols, uin
   SoA o;
   for (int k = 0; k < 4; k++) o.c[k] = h_out[k];
   const uint32_t rows = 1u << (log_size - log_blowup);
-  static thread_local NumeratorTerms terms;
-  for (uint32_t t0 = 0; t0 < n_terms; t0 += kMaxTerms) {
-    const uint32_t nt = std::min<uint32_t>(kMaxTerms, n_terms - t0);
-    terms.n = nt;
-    qm31 b_sum = qm31_make(0, 0, 0, 0);
-    for (uint32_t t = 0; t < nt; t++) {
-      const uint32_t* co = h_coeffs + 12 * (t0 + t);
-      terms.col[t] = h_cols[t0 + t];
-      b_sum = qm31_add(b_sum, qm31_make(co[4], co[5], co[6], co[7]));
-      terms.c[t] = qm31_make(co[8], co[9], co[10], co[11]);
-    }
-    terms.b_sum = b_sum;
+  for (uint32_t t0 = 0, nt; t0 < n_terms; t0 += nt) {
+    nt = std::min(kMmaTerms, n_terms - t0);
     // 64-row warps of 16-byte reads; small row counts in blocks of 64 threads, so that more SMs have one
     bool mma = nt >= kNumMmaMinTerms && rows >= kNumRows;
     for (int k = 0; k < 4; k++) mma = mma && aligned16(o.c[k]);
-    for (uint32_t t = 0; t < nt; t++) mma = mma && aligned16(terms.col[t]);
+    for (uint32_t t = 0; t < nt; t++) mma = mma && aligned16(h_cols[t0 + t]);
+    cudaStream_t st = to_stream(stream);
     if (mma) {
       const uint32_t threads = rows >= 152 * 2 * kNumThreads / 32 * kNumRows ? kNumThreads : 64;
       const uint32_t blocks = std::min<uint32_t>(rows / (threads / 32 * kNumRows), 152 * 2 * kNumThreads / threads);
-      numerators_mma_kernel<<<std::max(1u, blocks), threads, 0, to_stream(stream)>>>(terms, rows, o, t0 > 0);
+      numerators_mma_kernel<<<std::max(1u, blocks), threads, 0, st>>>(
+          numerator_terms<kMmaTerms>(h_cols + t0, h_coeffs + 12 * (size_t)t0, nt), rows, o, t0 > 0);
     } else {
-      numerators_kernel<<<grid_for(rows, 256), 256, 0, to_stream(stream)>>>(terms, rows, o, t0 > 0);
+      // every launch reads and writes the accumulators once more: as many terms as a launch's parameters hold
+      // (300 unaligned columns of 2^12 rows: 18.2 us in one launch, 19.6 in two)
+      nt = std::min(kMaxTerms, n_terms - t0);
+      const uint32_t* const* cols = h_cols + t0;
+      const uint32_t* coeffs = h_coeffs + 12 * (size_t)t0;
+      if (nt <= kMmaTerms)
+        numerators_kernel<<<grid_for(rows, 256), 256, 0, st>>>(numerator_terms<kMmaTerms>(cols, coeffs, nt), rows, o, t0 > 0);
+      else
+        numerators_kernel<<<grid_for(rows, 256), 256, 0, st>>>(numerator_terms<kMaxTerms>(cols, coeffs, nt), rows, o, t0 > 0);
     }
     CS_LAUNCHED("numerators_kernel");
   }

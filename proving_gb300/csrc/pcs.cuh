@@ -7,7 +7,8 @@
 
 namespace cs {
 
-constexpr uint32_t kMaxTerms = 256;   // numerator terms per launch (larger batches are split)
+constexpr uint32_t kMaxTerms = 512;   // numerator terms per launch (larger batches are split)
+constexpr uint32_t kMmaTerms = 256;   // the same on the tensor cores (their fragments are in shared memory)
 constexpr uint32_t kMaxPoints = 16;   // sample points per quotient launch
 
 struct GenPowersTable {
@@ -19,9 +20,10 @@ struct BaryColumns {
   const uint32_t* ptr[kMaxBatch];
 };
 
+template <uint32_t N>
 struct NumeratorTerms {
-  const uint32_t* col[kMaxTerms];
-  qm31 c[kMaxTerms];
+  const uint32_t* col[N];
+  qm31 c[N];
   qm31 b_sum;
   uint32_t n;
 };
