@@ -598,8 +598,13 @@ __global__ void numerators_kernel(const NumeratorTerms<N> terms, uint32_t rows, 
 constexpr int kNumThreads = 256;
 constexpr uint32_t kNumRows = 64;  // rows a warp: two loads a step for one set of coefficient fragments
 constexpr uint32_t kNumUnroll = 4;
-// With fewer terms a warp has too little in flight per pass over its rows: 24 terms of 2^20 rows take 33.4 us
-// here against 30.7 by multiply-adds, 26 of 2^22 101 against 115.
+// Fewer rows do not give every SM its 16 warps, and each block prepares the fragments of all terms first. Device us
+// by multiply-adds / here: 64 terms of 2^8 rows 5.3 / 5.7, of 2^16 6.6 / 7.1, of 2^17 10.3 / 12.5, of 2^18 16.3 /
+// 14.6; 256 terms of 2^17 39 / 58, of 2^18 65 / 54.
+constexpr uint32_t kNumMmaMinRows = 1u << 18;
+static_assert(kNumMmaMinRows >= 152 * 2 * (kNumThreads / 32) * kNumRows, "numerators: two full blocks an SM");
+// With fewer terms a warp has too little in flight per pass over its rows. 25 terms of 2^18 rows take 8.6 / 8.5 us,
+// of 2^22 107 / 94; 24 of 2^20 (out of L2) 30.7 / 33.4.
 constexpr uint32_t kNumMmaMinTerms = 25;
 
 __global__ void __launch_bounds__(kNumThreads, 2) numerators_mma_kernel(
@@ -1109,15 +1114,12 @@ extern "C" cs_status cs_accumulate_numerators(const uint32_t* const* h_cols, uin
   const uint32_t rows = 1u << (log_size - log_blowup);
   for (uint32_t t0 = 0, nt; t0 < n_terms; t0 += nt) {
     nt = std::min(kMmaTerms, n_terms - t0);
-    // 64-row warps of 16-byte reads; small row counts in blocks of 64 threads, so that more SMs have one
-    bool mma = nt >= kNumMmaMinTerms && rows >= kNumRows;
+    bool mma = nt >= kNumMmaMinTerms && rows >= kNumMmaMinRows;  // 16-byte reads
     for (int k = 0; k < 4; k++) mma = mma && aligned16(o.c[k]);
     for (uint32_t t = 0; t < nt; t++) mma = mma && aligned16(h_cols[t0 + t]);
     cudaStream_t st = to_stream(stream);
     if (mma) {
-      const uint32_t threads = rows >= 152 * 2 * kNumThreads / 32 * kNumRows ? kNumThreads : 64;
-      const uint32_t blocks = std::min<uint32_t>(rows / (threads / 32 * kNumRows), 152 * 2 * kNumThreads / threads);
-      numerators_mma_kernel<<<std::max(1u, blocks), threads, 0, st>>>(
+      numerators_mma_kernel<<<152 * 2, kNumThreads, 0, st>>>(
           numerator_terms<kMmaTerms>(h_cols + t0, h_coeffs + 12 * (size_t)t0, nt), rows, o, t0 > 0);
     } else {
       // every launch reads and writes the accumulators once more: as many terms as a launch's parameters hold
