@@ -692,6 +692,11 @@ __global__ void __launch_bounds__(kNumThreads, 2) numerators_mma_kernel(
 
 // ---------------------------------------------------------------- quotients
 
+// Fewer rows leave most of the chip idle at eight rows a thread, and a thread's chain counts. Device us, a row a
+// thread / eight: one point of 2^3 rows 5.0 / 5.7, of 2^15 6.4 / 6.9, of 2^16 8.5 / 6.8; four points of 2^10 8.2 /
+// 11.1, of 2^15 9.3 / 11.5, of 2^16 12.4 / 11.6.
+constexpr uint32_t kQuotientOctetsMinLog = 16;
+
 // Eight rows a thread (see octet_point): the denominators of a sample point are
 // C - X p_iy + Y p_ix with C = p_rx p_iy - p_ry p_ix, whose products the eight rows share, and their
 // norms are inverted together. 2^19 rows of one point: 48 -> 16 us (device time).
@@ -758,7 +763,7 @@ __global__ void __launch_bounds__(128) quotient_octets_kernel(const __grid_const
   }
 }
 
-// Subdomains of fewer than eight points, and columns that are not 8- / 16-byte aligned.
+// Subdomains of fewer than 2^16 points, and columns that are not 8- / 16-byte aligned.
 __global__ void quotients_kernel(const __grid_constant__ QuotientParams q, SoA out) {
   __shared__ cpoint tab[3][512];
   stage_tables(q.tables, tab);
@@ -842,7 +847,7 @@ cs_status quotients_on_subdomain(const QuotientParams& q, uint32_t* const out[4]
   SoA o;
   for (int k = 0; k < 4; k++) o.c[k] = out[k];
   const uint32_t rows = 1u << q.sub_log;
-  bool octets = q.sub_log >= 3;
+  bool octets = q.sub_log >= kQuotientOctetsMinLog;
   for (int k = 0; k < 4; k++) octets = octets && aligned16(out[k]);
   for (uint32_t p = 0; p < q.n_points; p++)
     for (int k = 0; k < 4; k++) octets = octets && (reinterpret_cast<uintptr_t>(q.acc[p].c[k]) & 7) == 0;
