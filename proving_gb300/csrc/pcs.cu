@@ -87,12 +87,12 @@ __device__ __forceinline__ cpoint table_point(const cpoint (*tab)[512], uint32_t
   return cpoint_add(cpoint_add(tab[0][jj & 511], tab[1][(jj >> 9) & 511]), tab[2][(jj >> 18) & 511]);
 }
 
-// Eight consecutive rows 8 q .. 8 q + 7 of a domain of 2^n >= 8 points share one point (x, y) up to
+// Eight consecutive rows 8 q .. 8 q + 7 of a domain of 2^n > 8 points share one point (x, y) up to
 // signs: rows 2 m and 2 m + 1 are conjugate, and the pairs m = 4 q + s hold the points of natural index
 // brev(q) + {0, 2, 1, 3}[s] 2^(n-3), where 2^(n-3) steps are the quarter turn (0, -1). Their pairs'
 // points are (x, +-y), (-x, -+y), (y, -+x), (-y, +-x).
 __device__ __forceinline__ cpoint octet_point(const cpoint (*tab)[512], uint32_t q, uint32_t log_n) {
-  return table_point(tab, log_n > 3 ? __brev(q) >> (35 - log_n) : 0);
+  return table_point(tab, __brev(q) >> (35 - log_n));
 }
 
 // The inverses of v[0..K-1] in place, by one inversion (Montgomery's trick); a zero's is zero, as
@@ -133,6 +133,9 @@ struct BaryParams {
 // -p.x the cancelled factor is zero only together with V_n(p) or is not zero.) An inverse takes 38
 // products; here eight rows share one point and one inversion of four norms. 2^20 weights: 53.8 -> 19.3 us
 // (device time; the columns written take 2.5).
+// Fewer rows leave most of the chip idle at eight rows a thread. Device us, a row a thread / eight: 2^5 rows 4.8 / 5.5,
+// 2^13 5.8 / 6.9, 2^15 6.6 / 7.0, 2^16 9.2 / 7.0.
+constexpr uint32_t kWeightPairsMinLog = 16;
 struct BaryPairParams {
   DomainTables tables;
   uint32_t log_n;
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(256) bary_weight_pairs_kernel(const __grid_con
   }
 }
 
-// Any point (and domains of fewer than eight points).
+// Any point, and domains of fewer than 2^16 points.
 __global__ void bary_weights_kernel(const __grid_constant__ BaryParams p, SoA out) {
   __shared__ cpoint tab[3][512];
   stage_tables(p.tables, tab);
@@ -979,7 +982,7 @@ extern "C" cs_status cs_barycentric_weights(uint32_t log_size, const uint32_t px
   }
   const qm31 norm = qm31_add(qm31_mul(p.px, p.px), qm31_mul(p.py, p.py));
   const bool on_circle = norm.a.a == 1 && (norm.a.b | norm.b.a | norm.b.b) == 0;
-  if (log_size >= 3 && aligned && on_circle) {
+  if (log_size >= kWeightPairsMinLog && aligned && on_circle) {
     static thread_local BaryPairParams r;
     r.tables = p.tables;
     r.log_n = log_size;
