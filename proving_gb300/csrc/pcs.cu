@@ -345,10 +345,12 @@ __global__ void __launch_bounds__(kBaryThreads, 3) bary_partial_kernel(const Bar
 // thousands of streams in flight cost DRAM more than the arithmetic saved. Bound: HBM.
 // 64 columns of 2^20: 82.5 -> 50.2 us (69.9 with the lanes' own loads); the mixed proof's 26 sets 3.99 ->
 // 2.44 ms (4.94).
-// A group always does the work of 16 columns: one column of 2^22 takes 54 us here and 22 by multiply-adds,
-// eight 55 and 59 (of 2^20: 22.2 both), seventeen 98 and 102.
 constexpr uint32_t kBaryMmaMinLog = 12;
-constexpr uint32_t kBaryMmaMinCols = 8;
+// From how many columns of 2^log rows on. A group always does the work of 16 columns, and from 2^18 rows to where
+// HBM bounds both forms the multiply-adds are the faster ones for few. Device us by multiply-adds / here, columns
+// of 2^20 or fewer in L2: 8 columns of 2^12 7.4 / 5.1, of 2^17 7.2 / 5.9, of 2^18 7.3 / 8.8, of 2^20 15.8 / 16.4,
+// of 2^22 52.3 / 49.4; 9 of 2^19 10.8 / 10.9, of 2^20 17.0 / 16.4; 12 of 2^18 9.0 / 8.8; 17 of 2^22 95 / 91.
+inline uint32_t bary_mma_min_cols(uint32_t log) { return log == 18 ? 12 : log > 18 && log < 22 ? 9 : 8; }
 constexpr int kBaryMmaCols = 16;           // columns per block (two groups of eight)
 constexpr uint32_t kBaryTile = 512;        // rows a tile, 64 a warp
 constexpr uint32_t kBaryStream = kBaryTile + 16;  // words: 64 bytes of padding keep eight columns on distinct banks
@@ -1023,7 +1025,7 @@ extern "C" cs_status cs_barycentric_eval(const uint32_t* const* h_cols, uint32_t
       cols.ptr[i] = h_cols[b0 + i];
     }
     const uint32_t n = 1u << log_size;
-    bool mma = log_size >= kBaryMmaMinLog && nb >= kBaryMmaMinCols;
+    bool mma = log_size >= kBaryMmaMinLog && nb >= bary_mma_min_cols(log_size);
     for (int k = 0; k < 4; k++) mma = mma && aligned16(w.c[k]);
     for (uint32_t i = 0; i < nb; i++) mma = mma && aligned16(cols.ptr[i]);
     const uint32_t groups = (nb + kBaryMmaCols - 1) / kBaryMmaCols;
