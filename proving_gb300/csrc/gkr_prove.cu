@@ -620,13 +620,14 @@ __device__ __forceinline__ qm31 warp_sum(qm31 v) {
   return v;
 }
 
-// One round of many terms over the whole chip: blockIdx.y is the instance (those that have not joined
-// or wait for their first round are counted all the same). The last block to finish ends the round.
+// One round of many terms over the whole chip: blockIdx.x is the instance (any number of them; those
+// that have not joined or wait for their first round are counted all the same), blockIdx.y its block.
+// The last block to finish ends the round.
 __global__ void __launch_bounds__(kRoundThreads) gkr_round_kernel(const GkrProgram g, uint32_t layer, uint32_t round) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ bool last;
   __shared__ qm31 part[4][kRoundThreads / 32];
-  const uint32_t i = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t i = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // how late the instance joins, from the table that no launch of the chain writes (InstState, which the
   // launch before this one writes back, may only be read after the wait)
   const LayerCols& L = g.cols[(size_t)layer * g.n_inst + i];
@@ -636,7 +637,7 @@ __global__ void __launch_bounds__(kRoundThreads) gkr_round_kernel(const GkrProgr
   const Block B = prefetch_block(g, smem, layer, round);
   if (delta <= round) {
     const Sums s = round_terms(L, round - delta, 1u << (layer - round - 1),
-                               blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, g.eq, 1u << (layer - 1),
+                               blockIdx.y * blockDim.x + threadIdx.x, gridDim.y * blockDim.x, g.eq, 1u << (layer - 1),
                                g.state->x);
     const qm31 w[4] = {warp_sum(s.a0), warp_sum(s.c0), warp_sum(s.a2), warp_sum(s.c2)};
     if (lane == 0)
@@ -645,7 +646,7 @@ __global__ void __launch_bounds__(kRoundThreads) gkr_round_kernel(const GkrProgr
     if (threadIdx.x < 4) {
       qm31 v = part[threadIdx.x][0];
       for (int k = 1; k < (int)kRoundThreads / 32; k++) v = qm31_add(v, part[threadIdx.x][k]);
-      q_put(g.partial + 16 * ((size_t)i * gridDim.x + blockIdx.x) + 4 * threadIdx.x, v);
+      q_put(g.partial + 16 * ((size_t)i * gridDim.y + blockIdx.y) + 4 * threadIdx.x, v);
       __threadfence();
     }
   }
@@ -659,8 +660,8 @@ __global__ void __launch_bounds__(kRoundThreads) gkr_round_kernel(const GkrProgr
     if (B.inst[j].delta > round) continue;
     // thread 4 b + k adds sum k of the blocks b, b + 32, ...
     qm31 v = q_zero();
-    for (uint32_t b = threadIdx.x >> 2; b < gridDim.x; b += kRoundThreads / 4) {
-      const uint4 u = __ldcg(reinterpret_cast<const uint4*>(g.partial + 16 * ((size_t)j * gridDim.x + b)) + (threadIdx.x & 3));
+    for (uint32_t b = threadIdx.x >> 2; b < gridDim.y; b += kRoundThreads / 4) {
+      const uint4 u = __ldcg(reinterpret_cast<const uint4*>(g.partial + 16 * ((size_t)j * gridDim.y + b)) + (threadIdx.x & 3));
       v = qm31_add(v, qm31_make(u.x, u.y, u.z, u.w));
     }
 #pragma unroll
@@ -1092,7 +1093,7 @@ cs_status gkr_prove_on_device(const std::vector<GkrInput>& inputs, uint32_t chan
     for (uint32_t r = 0; r + kTailRounds < l; r++) {
       const uint64_t terms = 1ull << (l - r - 1);
       const uint32_t blocks = (uint32_t)std::min<uint64_t>((terms + kRoundThreads - 1) / kRoundThreads, 152 * 8);
-      c = config(dim3(blocks, n_inst), kRoundThreads, round_bytes);
+      c = config(dim3(n_inst, blocks), kRoundThreads, round_bytes);
       CS_CUDA(cudaLaunchKernelEx(&c, gkr_round_kernel, (const GkrProgram)g, l, r));
       note_launch();
     }
