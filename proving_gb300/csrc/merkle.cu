@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kLeafThreads) merkle_leaves_kernel(const __gri
       const uint32_t base = b << 4;
       const bool last = p.is_final && b + 1 == p.block1;
       const uint32_t cnt = min(16u, p.n_cols - base);
-auto word = [&](int k) {
+      auto word = [&](int k) {
         if (READS == kLeafStrided) return __ldg(col + k * p.stride);
         const uint32_t c = base + k;
         return __ldg(p.cols[c] + (READS == kLeafLifted ? lift_index(x, p.level_log, p.log[c]) : x));

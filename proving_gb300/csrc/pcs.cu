@@ -397,10 +397,8 @@ __global__ void __launch_bounds__(kBaryThreads, 2) bary_mma_kernel(const __grid_
   const uint32_t bsel = (g & 3) | ((4 + (g & 3)) << 4);  // byte g & 3 of two words
   // a lane has, of column g of each group, every byte i of the column and bytes 2 (q & 1) and + 1 of the
   // weights' coordinates q / 2 and 2 + q / 2; byte i times byte j counts 2^(8 (i + j)) = 2^(8 (i + j) mod 31)
-  float acc[2][2][2][4];  // [group][bytes 0, 1 or 2, 3][coordinates 0, 1 or 2, 3][+ row 8][+ column 1]
+  float acc[2][2][2][4] = {};  // [group][bytes 0, 1 or 2, 3][coordinates 0, 1 or 2, 3][+ row 8][+ column 1]
   uint64_t sum[2][2] = {{0, 0}, {0, 0}};  // [group][coordinates]
-#pragma unroll
-  for (int i = 0; i < 32; i++) (&acc[0][0][0][0])[i] = 0;
   const uint32_t odd = q & 1;
   const uint32_t n_tiles = n / kBaryTile;
   uint32_t filled = 0;  // tiles summed since the last emptying: 64 rows each
@@ -624,8 +622,9 @@ __global__ void __launch_bounds__(kNumThreads, 2) numerators_mma_kernel(
     const uint32_t x0 = t < terms.n ? reinterpret_cast<const uint32_t*>(&terms.c[t])[n >> 1] : 0;
     const uint32_t x1 = m31_mul_pow2(x0, 8), x2 = m31_mul_pow2(x0, 16), x3 = m31_mul_pow2(x0, 24);
     const uint32_t lo = (n & 1) | ((4 + (n & 1)) << 4), hi = lo + 0x22;
-    frag[0][i] = make_uint4(byte_halves(__byte_perm(x0, x1, lo), 0x4140), byte_halves(__byte_perm(x2, x3, lo), 0x4140),
-                            byte_halves(__byte_perm(x0, x1, hi), 0x4140), byte_halves(__byte_perm(x2, x3, hi), 0x4140));
+    frag[i >> 5][i & 31] =
+        make_uint4(byte_halves(__byte_perm(x0, x1, lo), 0x4140), byte_halves(__byte_perm(x2, x3, lo), 0x4140),
+                   byte_halves(__byte_perm(x0, x1, hi), 0x4140), byte_halves(__byte_perm(x2, x3, hi), 0x4140));
   }
   for (uint32_t t = threadIdx.x; t < 4 * steps; t += blockDim.x) ptr[t] = t < terms.n ? terms.col[t] : nullptr;
   __syncthreads();
@@ -635,12 +634,8 @@ __global__ void __launch_bounds__(kNumThreads, 2) numerators_mma_kernel(
 #pragma unroll 1
   for (uint32_t r0 = (blockIdx.x * warps + warp) * kNumRows; r0 < rows; r0 += gridDim.x * warps * kNumRows) {
     const uint32_t row = r0 + 4 * g;
-    float acc[2][2][2][4];  // [32 rows][2 rows of four][bytes 0, 1 or 2, 3][+ row][+ byte]
-    uint64_t sum[2][4];
-#pragma unroll
-    for (int k = 0; k < 32; k++) (&acc[0][0][0][0])[k] = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) (&sum[0][0])[k] = 0;
+    float acc[2][2][2][4] = {};  // [32 rows][2 rows of four][bytes 0, 1 or 2, 3][+ row][+ byte]
+    uint64_t sum[2][4] = {};
 #pragma unroll 1
     for (uint32_t s0 = 0; s0 < steps; s0 += kNumUnroll) {
       uint4 v[kNumUnroll][2];
