@@ -49,7 +49,7 @@ def _ptr_table(ts) -> ctypes.Array:
 
 
 def _u32_table(vals) -> ctypes.Array:
-    words = vals.tolist() if isinstance(vals, np.ndarray) else list(map(int, vals))
+    words = list(map(int, vals.tolist() if isinstance(vals, np.ndarray) else vals))
     return (ctypes.c_uint32 * max(1, len(words)))(*words)
 
 
