@@ -138,9 +138,7 @@ __global__ void merkle_node_kernel(const uint32_t* __restrict__ prev, uint32_t l
 // nodes of S = 10 need, 12 for 8 with S = 8.
 constexpr uint32_t kSubtreeMaxLog = 10;
 
-template <bool CHAIN>
-__global__ void __launch_bounds__(256) merkle_subtree_kernel(uint32_t* layer, uint32_t log_in, uint32_t S,
-                                                             uint32_t one) {
+__global__ void __launch_bounds__(256) merkle_subtree_kernel(uint32_t* layer, uint32_t log_in, uint32_t S) {
   __shared__ __align__(8) uint32_t even[8][1u << (kSubtreeMaxLog - 1)];  // levels 1, 3, ...
   __shared__ __align__(8) uint32_t odd[8][1u << (kSubtreeMaxLog - 2)];   // levels 2, 4, ...
   for (uint32_t k = 1; k <= S; k++) {
@@ -169,7 +167,7 @@ __global__ void __launch_bounds__(256) merkle_subtree_kernel(uint32_t* layer, ui
         }
       }
       b2s_init(h);
-      b2s_compress<CHAIN>(h, m, 64, 0, true, one);
+      b2s_compress<true>(h, m, 64, 0, true);
 #pragma unroll
       for (int w = 0; w < 8; w++) {
         if (k & 1)
@@ -363,12 +361,9 @@ cs_status merkle_layers(uint32_t* d_layers, uint32_t L, cudaStream_t st) {
     }
     const uint32_t S = subtree_levels(k);
     const uint32_t threads = std::max(32u, std::min(256u, 1u << (S - 1)));
-    const uint32_t blocks = 1u << (k - S);
-    // two blocks an SM or more: the compression's throughput form
-    if (blocks > 2 * 152)
-      merkle_subtree_kernel<false><<<blocks, threads, 0, st>>>(cur, k, S, 1u);
-    else
-      merkle_subtree_kernel<true><<<blocks, threads, 0, st>>>(cur, k, S, 1u);
+    // at most 2^8 blocks (below 19), for which the low-latency compression is the faster form: trees of 2^17 leaves
+    // 32.2 us against 39.3 by the multiply-adds (128 blocks here), of 2^18 50.0 against 50.3 (256)
+    merkle_subtree_kernel<<<1u << (k - S), threads, 0, st>>>(cur, k, S);
     CS_LAUNCHED("merkle_subtree_kernel");
     cur += 8 * (((size_t)2 << k) - ((size_t)2 << (k - S)));
     k -= S;
