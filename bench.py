@@ -56,9 +56,9 @@ def workload_name():
 
 # DRAM bytes (read + write) measured with ncu on the 256 x 2^20 workload
 # (profiles/launch_list_commit_stage_256x2^20.md): one merkle_leaves_kernel launch, and the two
-# FFT pass launches of one evaluate
-LEAVES_TRAFFIC_BYTES = 4425.2e6
-EVALUATE_TRAFFIC_BYTES = 13935.0e6
+# launches of one evaluate (fft_strided_kernel 5,311.3 MB, fft_contig_kernel 8,800.7 MB)
+LEAVES_TRAFFIC_BYTES = 4425.5e6
+EVALUATE_TRAFFIC_BYTES = 14112.0e6
 
 
 def set_shape(n_cols: int, log_rows: int):

@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(tile_max_threads<T, OUTER>(), tile_min_blocks<
   }
 }
 
-// ---- passes of up to 10 layers: tiles go between global memory and registers directly ----
+// ---- passes of up to 11 layers: tiles go between global memory and registers directly ----
 //
 // The same two register stages, with less around them than fft_tile_kernel. A thread's first
 // stage loads its values straight from global memory and its last stage stores them straight from
@@ -367,8 +367,8 @@ __global__ void __launch_bounds__(tile_max_threads<T, OUTER>(), tile_min_blocks<
 // passes run at 12.4 (contiguous) and 13.9-14.7 cycles a butterfly with DRAM 20-45% busy, against
 // 15.8-17.2 for tiles staged through shared memory on both sides of the stages (four block
 // barriers, twice the shared accesses, per-word address arithmetic). Measured, CUDA events:
-// 256 columns of 2^20 interpolate 1.33 -> 1.04 ms and evaluate onto 2^22 4.71 -> 3.69 ms; one
-// column of 2^24 138 -> 100 and 257 -> 178 us; 32 columns of 2^22 743 -> 640 and 1408 -> 1153 us.
+// 256 columns of 2^20 interpolate 1.26 -> 0.98 ms and evaluate onto 2^22 4.59 -> 3.55 ms; one
+// column of 2^24 124 -> 92 and 239 -> 161 us; 32 columns of 2^22 743 -> 640 and 1408 -> 1153 us.
 // Passes of 11 layers hold 64 values a thread (two stages of 5 and 6 layers, 512 threads an SM);
 // contiguous passes of up to 5 layers, strided ones of up to 3 and the 12-layer pass stay with
 // fft_tile_kernel (a 12-layer pass would need a third stage; 1000 columns of 2^12 measured 293 us
@@ -607,8 +607,8 @@ __global__ void __launch_bounds__(32 * kContigWarps, direct_min_blocks<T - T / 2
   }
 }
 
-// Layers [lo, lo + T), lo >= 3: a block owns the 2^T values of 8 neighbouring groups (32-byte runs
-// in memory), one (group, stage row) a thread.
+// Layers [lo, lo + T), lo >= EB: a block owns the 2^T values of 2^EB = 8 or 16 neighbouring groups
+// (32- or 64-byte runs in memory), one (group, stage row) a thread.
 template <bool INV, int T, int EB>
 __global__ void __launch_bounds__((1 << EB) << (T / 2), direct_min_blocks<T - T / 2>((1 << EB) << (T / 2)))
     fft_strided_kernel(const __grid_constant__ FftBatch batch, const FftPass p) {
@@ -842,7 +842,7 @@ std::vector<PassPlan> plan_passes(bool inverse, uint32_t log_n, uint32_t n_layer
       const uint32_t want = TA >= 8 ? 0 : 8 - TA;
       pp.c = std::min(want, log_n - pp.hi);
     } else {
-      pp.outer = 0;  // strided tile: 8 neighbouring groups (32-byte runs in HBM)
+      pp.outer = 0;  // strided tile: 8 neighbouring groups or more (32-byte runs in HBM)
       pp.c = kStridedC;
     }
     plan.push_back(pp);

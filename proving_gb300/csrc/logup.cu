@@ -7,8 +7,9 @@
 // circle-domain index k / 2 (k even) or n/2 + (n - 1 - k) / 2 (k odd)
 // (crates/stwo/src/core/utils.rs:177-188), stored at its bit reversal.
 //
-// Several columns of any sizes go through three launches per batch, with no
-// host round trip between them and with every HBM access coalesced. With
+// Several columns of any sizes go through three launches per batch (and a
+// fourth for its columns of at most 2^9 rows), with no host round trip
+// between them and with every HBM access coalesced. With
 // c the natural circle-domain index of storage position p (c = bitrev(p)),
 // P the inclusive prefix sum of the fractions g in natural order and
 // T = P(n - 1), the unshifted coset-order running sum at p is
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(kTileThreads) outputs_kernel(const SumBatch b)
   }
 }
 
-// Runs the three launches over columns [0, n) of the tables; claimed sums to d_claimed (4 words each).
+// Runs the launches over columns [0, n) of the tables; claimed sums to d_claimed (4 words each).
 cs_status scan_columns(const uint32_t* const* values, const Q4* outs, const uint32_t* log_sizes, uint32_t n,
                        const qm31& z, uint32_t* d_claimed, cudaStream_t st) {
   uint64_t all_runs = 0;  // run totals, then 32 segment offsets, per column of 2^10 or more rows
